@@ -352,8 +352,15 @@ STPGB_API int stpgb_hydraulic_erosion(float* heightmap, const stpgb_nn_info* nn,
  * STPGB_EROSION_POINTWISE keeps the point-by-point kernels.
  * STPGB_EROSION_EXACT_CLAMP erodes each point by compare-and-swap instead, so
  * racing droplets never remove more than a cell holds (closer to the serial
- * algorithm, slower).  No counterpart in the reference. */
-enum { STPGB_EROSION_EXACT_CLAMP = 1, STPGB_EROSION_POINTWISE = 2 };
+ * algorithm, slower).  Where the droplets could erode 10^9 brush points or
+ * more, the default (lanes_per_droplet = 0, one droplet per group, no flag)
+ * erodes the map in tiles held in shared memory instead, with up to 64 MiB of
+ * device memory kept between such calls (more is given back); it does so for
+ * any size with STPGB_EROSION_TILES.  A call on a stream that is being
+ * captured, a map with values that are not finite or a largest magnitude above
+ * 64 times the mean one, a brush radius above 6 and lifetimes above 1024 steps
+ * keep to the kernels above.  No counterpart in the reference. */
+enum { STPGB_EROSION_EXACT_CLAMP = 1, STPGB_EROSION_POINTWISE = 2, STPGB_EROSION_TILES = 4 };
 
 /* The kernel variant the default (lanes_per_droplet = 0) of
  * stpgb_hydraulic_erosion_ex takes for a brush of `brush_radius` and
@@ -743,7 +750,10 @@ STPGB_API int stpgb_batch_tune(stpgb_batch* batch);
  * blocks, 0 = point by point; 1 lane with rows = the warp-cooperative kernel)
  * in use, and the autotuner's erosion time in ms per candidate: 36 floats,
  * index 18*rows + 3*log2(lanes) + {0, 1, 2} for 1, 2, 4 droplets per group
- * (0 = not tried).  Any output pointer may be NULL. */
+ * (0 = not tried).  A group that erodes in shared-memory tiles
+ * (STPGB_EROSION_TILES), because they were faster or, without tuning, because
+ * its droplets are many, reports the fastest of these variants beside, which
+ * erodes the maps the tiles do not take.  Any output pointer may be NULL. */
 STPGB_API int stpgb_batch_tuning(const stpgb_batch* batch, uint32_t* lanes_per_droplet,
 	uint32_t* droplets_per_group, uint32_t* vector_rows, float* erosion_ms);
 

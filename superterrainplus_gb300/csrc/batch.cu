@@ -82,6 +82,11 @@ struct ErosionGroup {
 	uint32_t interleave_extra = 0u;
 	// autotuner's erosion time per candidate, [rows 0, 1][lanes 1..32][droplets 1, 2, 4] (0 = not tried)
 	float tune_ms[36] = {};
+	// the tiles of erosion_tile.cu: their side (0 where they do not take a job of the group), and
+	// whether the group is eroded in them rather than by the variant above
+	uint32_t tile = 0u;
+	bool tiled = false;
+	unsigned char* tile_ws = nullptr;
 
 	void add(const ErosionJob& e, const uint32_t radius, const double d, const double f) {
 		h.push_back(e);
@@ -107,9 +112,17 @@ struct ErosionGroup {
 	}
 
 	int launch(cudaStream_t s) const {
+		const uint32_t* taken = nullptr;
+		if (tiled) {
+			STPGB_TRY(erosion_tile_launch(h.data(), jobs, static_cast<uint32_t>(h.size()), tile, tile_ws, &taken, s));
+		}
 		return erosion_launch(jobs, h[0], static_cast<uint32_t>(h.size()), max_count, max_brush, s, lanes, false, dpg,
 			rows, erosion_rows_wide(min_radius), erosion_rows_atomic(min_radius, lanes),
-			coop_interleave());
+			coop_interleave(), taken);
+	}
+
+	uint32_t kernels() const {
+		return 1u + (tiled ? erosion_tile_kernels(h.data(), static_cast<uint32_t>(h.size()), tile) : 0u);
 	}
 
 	uint32_t coop_interleave() const {
@@ -214,6 +227,11 @@ struct stpgb_batch {
 				 static_cast<void*>(fmt_jobs) }) {
 			if (p) {
 				cudaFree(p);
+			}
+		}
+		for (const ErosionGroup& g : grp) {
+			if (g.tile_ws) {
+				cudaFree(g.tile_ws);
 			}
 		}
 		if (fork) {
@@ -359,6 +377,7 @@ struct stpgb_batch {
 			float best = 0.0f;
 			uint32_t best_lanes = G.lanes, best_dpg = G.dpg, best_extra = 0u;
 			G.interleave_extra = 0u;
+			G.tiled = false;
 			bool best_rows = G.rows;
 			for (int c = 0; c < 36 && rc == STPGB_OK; c++) {
 				const bool cr = c >= 18;
@@ -447,6 +466,26 @@ struct stpgb_batch {
 				}
 				G.interleave_extra = best_extra;
 			}
+			// the tiles, where they take the group, against the fastest of the above
+			if (rc == STPGB_OK && G.tile_ws) {
+				G.tiled = true;
+				float t = 0.0f;
+				for (int rep = 0; rep < 2 && rc == STPGB_OK; rep++) {
+					rc = stage(1u, s);
+					if (rc == STPGB_OK) {
+						cudaEventRecord(e0, s);
+						rc = G.launch(s);
+						cudaEventRecord(e1, s);
+					}
+					if (cudaStreamSynchronize(s) != cudaSuccess) {
+						rc = cuda_fail(cudaGetLastError(), "autotune");
+					}
+					float ms = 0.0f;
+					cudaEventElapsedTime(&ms, e0, e1);
+					t = rep == 0 ? ms : std::min(t, ms);
+				}
+				G.tiled = t < best;
+			}
 		}
 		cudaEventDestroy(e0);
 		cudaEventDestroy(e1);
@@ -470,8 +509,17 @@ struct stpgb_batch {
 			const ErosionJob& e = ero_h[n];
 			const ErosionGroup& G = grp[group_of[n]];
 			STPGB_CUDA_TRY(cudaMemsetAsync(e.residual, 0, sizeof(double), s));
-			STPGB_TRY(erosion_launch(nullptr, e, 1u, e.count, e.brush_size, s, G.lanes, false, G.dpg, G.rows,
-				erosion_rows_wide(G.min_radius), erosion_rows_atomic(G.min_radius, G.lanes)));
+			void* tiles = nullptr;
+			const uint32_t* taken = nullptr;
+			if (G.tiled) {
+				STPGB_TRY(erosion_tile_call(e, false, &tiles, &taken, s));
+			}
+			const int erc = erosion_launch(nullptr, e, 1u, e.count, e.brush_size, s, G.lanes, false, G.dpg, G.rows,
+				erosion_rows_wide(G.min_radius), erosion_rows_atomic(G.min_radius, G.lanes), 1u, taken);
+			if (tiles) {
+				STPGB_CUDA_TRY(cudaFreeAsync(tiles, s));
+			}
+			STPGB_TRY(erc);
 			const FormatJob& f = fmt_h[n];
 			STPGB_TRY(format_launch(f.in, f.in_pitch, f.out, f.out_pitch, f.W, f.H, s));
 			STPGB_CUDA_TRY(cudaStreamSynchronize(s));
@@ -691,6 +739,24 @@ int stpgb_batch_create(const stpgb_batch_request* requests, uint32_t count, cons
 		STPGB_TRY(upload(b->grp[g].jobs, b->grp[g].h));
 	}
 	STPGB_TRY(upload(b->fmt_jobs, b->fmt_h));
+	// the tiles' workspaces, where the tiles pay and the budget has room for them
+	for (uint32_t g = 0u; g < b->ngroups; g++) {
+		ErosionGroup& G = b->grp[g];
+		const uint32_t njobs = static_cast<uint32_t>(G.h.size()), side = erosion_tile_side(G.h.data(), njobs);
+		const size_t bytes = side ? erosion_tile_bytes(G.h.data(), njobs, side) : 0u;
+		if (side == 0u || !erosion_tile_pays(G.h.data(), njobs) || (hbm_budget != 0u && b->bytes + bytes > hbm_budget)) {
+			continue;
+		}
+		if (cudaMalloc(&G.tile_ws, bytes) != cudaSuccess) {
+			cudaGetLastError();
+			G.tile_ws = nullptr;
+			continue;
+		}
+		b->bytes += bytes;
+		G.tile = side;
+		G.tiled = true;
+		STPGB_TRY(erosion_tile_prepare(G.h.data(), njobs, side, G.tile_ws));
+	}
 	if (b->ngroups > 1u) {
 		STPGB_CUDA_TRY(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
 		for (uint32_t g = 1u; g < b->ngroups; g++) {
@@ -926,8 +992,11 @@ int stpgb_batch_kernels_per_run(const stpgb_batch* b, uint32_t* kernels) {
 		*kernels = k;
 		return STPGB_OK;
 	}
-	// without a graph: the filter's nine launches, noise, one erosion launch per group, format
-	*kernels = 9u + 1u + b->ngroups + 1u;
+	// without a graph: the filter's nine launches, noise, the erosion groups' launches, format
+	*kernels = 9u + 1u + 1u;
+	for (uint32_t g = 0u; g < b->ngroups; g++) {
+		*kernels += b->grp[g].kernels();
+	}
 	return STPGB_OK;
 }
 

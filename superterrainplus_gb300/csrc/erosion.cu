@@ -97,8 +97,11 @@ constexpr uint32_t kCasRetries = 16u;
 // which gives every lane the same total.
 template<uint32_t G, bool ExactClamp>
 __global__ void __launch_bounds__(kErodeBlock) erosion_kernel(const ErosionJob* __restrict__ jobs,
-	const ErosionJob single) {
+	const ErosionJob single, const uint32_t* __restrict__ gate) {
 	const ErosionJob& J = jobs ? jobs[blockIdx.y] : single;
+	if (gate && gate[blockIdx.y] != 0u) {
+		return; // eroded in tiles
+	}
 	extern __shared__ unsigned char esm[];
 	int32_t* const bidx = reinterpret_cast<int32_t*>(esm);
 	float* const bw = reinterpret_cast<float*>(esm) + J.brush_size;
@@ -295,9 +298,12 @@ template<uint32_t G, uint32_t K>
 // 8 resident blocks of 128 threads (64 registers) for two droplets per group:
 // residency, not the few spilled registers, bounds this chain-latency kernel.
 __global__ void __launch_bounds__(kErodeBlock, K == 2u ? 8 : 1) erosion_multi_kernel(const ErosionJob* __restrict__ jobs,
-	const ErosionJob single) {
+	const ErosionJob single, const uint32_t* __restrict__ gate) {
 	static_assert(G >= 4u && K >= 2u, "one corner per lane needs four lanes");
 	const ErosionJob& J = jobs ? jobs[blockIdx.y] : single;
+	if (gate && gate[blockIdx.y] != 0u) {
+		return;
+	}
 	extern __shared__ unsigned char esm[];
 	int32_t* const bidx = reinterpret_cast<int32_t*>(esm);
 	float* const bw = reinterpret_cast<float*>(esm) + J.brush_size;
@@ -595,9 +601,13 @@ __device__ __forceinline__ void deposit_row(float* const c0, const float d0, con
 // fast for two lanes and one droplet and 6-15 % slower for the others).
 template<uint32_t G, uint32_t K>
 __global__ void __launch_bounds__(kErodeBlock, K == 2u ? 8 : 9) erosion_rows_kernel(const ErosionJob* __restrict__ jobs,
-	const ErosionJob single, const uint32_t resident, const bool wide, const bool atomic_brush) {
+	const ErosionJob single, const uint32_t resident, const bool wide, const bool atomic_brush,
+	const uint32_t* __restrict__ gate) {
 	static_assert((G == 2u || G == 4u) && (K == 1u || K == 2u), "2 or 4 lanes, 1 or 2 droplets");
 	const ErosionJob& J = jobs ? jobs[blockIdx.y] : single;
+	if (gate && gate[blockIdx.y] != 0u) {
+		return;
+	}
 	extern __shared__ unsigned char esm[];
 	int32_t* const bidx = reinterpret_cast<int32_t*>(esm);
 	float* const bw = reinterpret_cast<float*>(esm) + J.brush_size;
@@ -970,7 +980,7 @@ constexpr uint32_t kCoopBlocksPerSM = 8u;
 
 __global__ void __launch_bounds__(kErodeBlock, kCoopBlocksPerSM) erosion_coop_kernel(const ErosionJob* __restrict__ jobs,
 	const ErosionJob single, const uint32_t runcap, const uint32_t njobs, const uint32_t interleave,
-	const uint32_t blocks_per_job) {
+	const uint32_t blocks_per_job, const uint32_t* __restrict__ gate) {
 	constexpr uint32_t kWarps = kErodeBlock / 32u;
 	uint32_t job = 0u, bx = blockIdx.x;
 	if (jobs) {
@@ -981,6 +991,9 @@ __global__ void __launch_bounds__(kErodeBlock, kCoopBlocksPerSM) erosion_coop_ke
 		bx = within / qn;
 	}
 	const ErosionJob& J = jobs ? jobs[job] : single;
+	if (gate && gate[job] != 0u) {
+		return;
+	}
 	extern __shared__ __align__(16) unsigned char esm[];
 	int32_t* const bidx = reinterpret_cast<int32_t*>(esm);
 	float* const bw = reinterpret_cast<float*>(esm) + J.brush_size;
@@ -1421,7 +1434,8 @@ RainParams rain_params(const stpgb_raindrop_setting& s) {
 
 int erosion_launch(const ErosionJob* jobs, const ErosionJob& single, uint32_t njobs, uint32_t max_count,
 	uint32_t max_brush, cudaStream_t stream, uint32_t lanes_per_droplet, bool exact_clamp,
-	uint32_t droplets_per_group, bool vector_rows, bool wide_trips, bool atomic_brush, uint32_t interleave) {
+	uint32_t droplets_per_group, bool vector_rows, bool wide_trips, bool atomic_brush, uint32_t interleave,
+	const uint32_t* gate) {
 	if (max_count == 0u || njobs == 0u) {
 		return STPGB_OK;
 	}
@@ -1447,7 +1461,7 @@ int erosion_launch(const ErosionJob* jobs, const ErosionJob& single, uint32_t nj
 		}
 		const uint32_t q = jobs ? std::max(1u, std::min(interleave, njobs)) : 1u;
 		erosion_coop_kernel<<<static_cast<uint32_t>(per_job * njobs), kErodeBlock, csmem, stream>>>(jobs, single,
-			runcap, njobs, q, static_cast<uint32_t>(per_job));
+			runcap, njobs, q, static_cast<uint32_t>(per_job), gate);
 		STPGB_CUDA_TRY(cudaGetLastError());
 		return STPGB_OK;
 	}
@@ -1466,7 +1480,7 @@ int erosion_launch(const ErosionJob* jobs, const ErosionJob& single, uint32_t nj
 					static_cast<int>(rsmem)));
 			}
 			kernel<<<rgrid, kErodeBlock, rsmem, stream>>>(jobs, single,
-				erosion_resident_droplets(lanes_per_droplet, droplets_per_group), wide_trips, atomic_brush);
+				erosion_resident_droplets(lanes_per_droplet, droplets_per_group), wide_trips, atomic_brush, gate);
 			STPGB_CUDA_TRY(cudaGetLastError());
 			return STPGB_OK;
 		};
@@ -1496,7 +1510,7 @@ int erosion_launch(const ErosionJob* jobs, const ErosionJob& single, uint32_t nj
 				STPGB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
 					static_cast<int>(smem)));
 			}
-			kernel<<<mgrid, kErodeBlock, smem, stream>>>(jobs, single);
+			kernel<<<mgrid, kErodeBlock, smem, stream>>>(jobs, single, gate);
 			STPGB_CUDA_TRY(cudaGetLastError());
 			return STPGB_OK;
 		};
@@ -1527,7 +1541,7 @@ int erosion_launch(const ErosionJob* jobs, const ErosionJob& single, uint32_t nj
 		if (smem > 48u * 1024u) {
 			STPGB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
 		}
-		kernel<<<grid, kErodeBlock, smem, stream>>>(jobs, single);
+		kernel<<<grid, kErodeBlock, smem, stream>>>(jobs, single, gate);
 		STPGB_CUDA_TRY(cudaGetLastError());
 		return STPGB_OK;
 	};
@@ -1628,15 +1642,25 @@ int stpgb_hydraulic_erosion_ex(float* heightmap, const stpgb_nn_info* nn, const 
 	uint32_t lanes = lanes_per_droplet, dpg = droplets_per_group == 0u ? 1u : droplets_per_group;
 	const double area = static_cast<double>(nn->MapSize[0]) * nn->MapSize[1];
 	const double density = static_cast<double>(count) / area;
+	void* tiles = nullptr;
+	const uint32_t* gate = nullptr;
+	const cudaStream_t s = as_stream(stream);
 	if (lanes == 0u) {
 		const ErosionChoice c = erosion_choice(setting->ErosionBrushRadius, brush_size, density,
 			erosion_in_flight(count, area), rows);
 		lanes = c.lanes;
+		if (!exact && dpg == 1u && (flags & STPGB_EROSION_POINTWISE) == 0u) {
+			STPGB_TRY(erosion_tile_call(job, (flags & STPGB_EROSION_TILES) != 0u, &tiles, &gate, s));
+		}
 		rows = c.rows;
 	}
-	return erosion_launch(nullptr, job, 1u, count, brush_size, as_stream(stream), lanes, exact, dpg, rows,
+	const int rc = erosion_launch(nullptr, job, 1u, count, brush_size, s, lanes, exact, dpg, rows,
 		erosion_rows_wide(setting->ErosionBrushRadius),
-		erosion_rows_atomic(setting->ErosionBrushRadius, lanes));
+		erosion_rows_atomic(setting->ErosionBrushRadius, lanes), 1u, gate);
+	if (tiles) {
+		STPGB_CUDA_TRY(cudaFreeAsync(tiles, s));
+	}
+	return rc;
 }
 
 int stpgb_erosion_choice(uint32_t brush_radius, uint32_t droplets, uint32_t area, uint32_t* lanes_per_droplet,

@@ -56,7 +56,7 @@ RainParams rain_params(const stpgb_raindrop_setting& s);
 int erosion_launch(const ErosionJob* jobs, const ErosionJob& single, uint32_t njobs, uint32_t max_count,
 	uint32_t max_brush, cudaStream_t stream, uint32_t lanes_per_droplet, bool exact_clamp = false,
 	uint32_t droplets_per_group = 1u, bool vector_rows = false, bool wide_trips = false, bool atomic_brush = false,
-	uint32_t interleave = 1u);
+	uint32_t interleave = 1u, const uint32_t* gate = nullptr);
 // Jobs a warp-cooperative launch interleaves: enough that each keeps at most
 // kCoopInterleaveInFlight droplets in flight per pixel, with the maps of the
 // interleaved jobs together in half of the L2.
@@ -146,6 +146,30 @@ struct ErosionChoice {
 // droplets per pixel of the start area, `in_flight` of them at once.
 ErosionChoice erosion_choice(uint32_t radius, uint32_t brush_size, double density, double in_flight,
 	bool rows_allowed);
+
+// Erosion in shared-memory tiles (erosion_tile.cu).  `jobs` / `host_jobs` are
+// host copies; `device_jobs` the same on the device, or null for one job.
+// Droplets that take more steps than this stay with the kernels above: a phase
+// of the tiles may hold a droplet until it has taken all of them.
+constexpr uint32_t kTileMaxSteps = 1024u;
+// Whether the tiles are the faster way for these jobs.
+bool erosion_tile_pays(const ErosionJob* jobs, uint32_t njobs);
+// The tile side for a launch over these jobs, 0 where the tiles do not take one of them.
+uint32_t erosion_tile_side(const ErosionJob* jobs, uint32_t njobs);
+// Workspace of a launch, and what it holds from launch to launch (more than one job only).
+size_t erosion_tile_bytes(const ErosionJob* jobs, uint32_t njobs, uint32_t side);
+int erosion_tile_prepare(const ErosionJob* jobs, uint32_t njobs, uint32_t side, void* workspace);
+// `taken`: per job (device) 1 if its map and brush suit the tiles and it was eroded, 0 if it is
+// untouched and left to erosion_launch with `gate` = taken.
+int erosion_tile_launch(const ErosionJob* host_jobs, const ErosionJob* device_jobs, uint32_t njobs, uint32_t side,
+	void* workspace, const uint32_t** taken, cudaStream_t stream);
+// kernels of such a launch
+uint32_t erosion_tile_kernels(const ErosionJob* jobs, uint32_t njobs, uint32_t side);
+// The same for one job with a workspace of the library's own, returned in `workspace` for the
+// caller to free on `stream` (cudaFreeAsync); null, and nothing launched, where the tiles do not
+// pay (unless `force`) or do not take the job, the stream is being captured or the workspace
+// cannot be had.
+int erosion_tile_call(const ErosionJob& job, bool force, void** workspace, const uint32_t** taken, cudaStream_t stream);
 
 int format_launch(const float* in, uint64_t in_pitch, uint16_t* out, uint64_t out_pitch, uint32_t W, uint32_t H,
 	cudaStream_t stream);
