@@ -41,7 +41,7 @@ constexpr uint32_t kVAhead = 8u;
 constexpr uint32_t kHBlock = 32u;
 // columns (rows) a segment's start sweep loads ahead of their use
 constexpr uint32_t kSweepAhead = 8u;
-constexpr uint32_t kScanBlock = 256u;
+constexpr uint32_t kScanBlock = 1024u;
 // consecutive (row, segment) counts a scan thread takes per pass
 constexpr uint32_t kScanPer = 16u;
 // threads per SM the segmented passes aim for
@@ -183,7 +183,9 @@ __global__ void __launch_bounds__(kVBlock) shf_vertical(const ShfJob* __restrict
 			}
 		});
 		// upward sweep: extend each run while its occurrences stay within 2r+1
-		// rows; the samples are loaded kSweepAhead rows ahead
+		// rows, until all runs but one are known to have started (that one
+		// started above the others, wherever); the samples are loaded
+		// kSweepAhead rows ahead
 		uint32_t open = n;
 		uint32_t sv[kSweepAhead];
 		const int q_top = static_cast<int>(y_a) - r - 1;
@@ -193,11 +195,11 @@ __global__ void __launch_bounds__(kVBlock) shf_vertical(const ShfJob* __restrict
 				sv[u] = at(q_top - static_cast<int>(u));
 			}
 		}
-		for (int q0 = q_top; q0 >= -r && open > 0u; q0 -= static_cast<int>(kSweepAhead)) {
+		for (int q0 = q_top; q0 >= -r && open > 1u; q0 -= static_cast<int>(kSweepAhead)) {
 #pragma unroll
 			for (uint32_t u = 0u; u < kSweepAhead; u++) {
 				const int q = q0 - static_cast<int>(u);
-				if (q >= -r && open > 0u) {
+				if (q >= -r && open > 1u) {
 					const uint32_t v = sv[u], qk = static_cast<uint32_t>(q + r);
 					if (q - static_cast<int>(kSweepAhead) >= -r) {
 						sv[u] = at(q - static_cast<int>(kSweepAhead));
@@ -397,7 +399,8 @@ __global__ void __launch_bounds__(kHBlock) shf_horizontal(const ShfJob* __restri
 				key[(n - 1u) * kHBlock] = (kc << 12) | j;
 			}
 		});
-		// leftward sweep: extend each run while its columns stay within 2r+1;
+		// leftward sweep: extend each run while its columns stay within 2r+1,
+		// until all but one are known to have started;
 		// the columns' data is loaded kSweepAhead columns ahead (their loads do
 		// not depend on the sweep), so the sweep is not a chain of round trips
 		uint32_t open = n;
@@ -408,11 +411,11 @@ __global__ void __launch_bounds__(kHBlock) shf_horizontal(const ShfJob* __restri
 				sw[u] = fetch(x_a - 1u - u);
 			}
 		}
-		for (int kc0 = static_cast<int>(x_a) - 1; kc0 >= 0 && open > 0u; kc0 -= static_cast<int>(kSweepAhead)) {
+		for (int kc0 = static_cast<int>(x_a) - 1; kc0 >= 0 && open > 1u; kc0 -= static_cast<int>(kSweepAhead)) {
 #pragma unroll
 			for (uint32_t u = 0u; u < kSweepAhead; u++) {
 				const int kc = kc0 - static_cast<int>(u);
-				if (kc >= 0 && open > 0u) {
+				if (kc >= 0 && open > 1u) {
 					const ColData c = sw[u];
 					if (kc >= static_cast<int>(kSweepAhead)) {
 						sw[u] = fetch(static_cast<uint32_t>(kc) - kSweepAhead);

@@ -16,7 +16,7 @@
 //   shf_palette       block per (32-row tile of the read region, job):
 //                     distinct values through a 65536-bit map in shared
 //                     memory.
-//   shf_route         thread per job: the path (few-values or general).
+//   shf_route         warp per job: the path (few-values or general).
 //   shf_vertical_fast thread per column: slides the column's vertical
 //                     histogram down all rows and writes it to row-major
 //                     planes in the job's vbuf.
@@ -33,7 +33,9 @@ using namespace shfx;
 
 namespace {
 
-constexpr uint32_t kPaletteBlock = 256u;
+constexpr uint32_t kPaletteBlock = 512u;
+// samples of a row a lane loads together
+constexpr uint32_t kPaletteAhead = 8u;
 constexpr uint32_t kVertBlock = 64u;
 constexpr uint32_t kRowBlock = 64u;
 // rows of the vertical slide whose samples are loaded ahead of their use
@@ -46,19 +48,55 @@ constexpr uint64_t kSlideRowsPerSM = 256u;
 
 // ---------------------------------------------------------------- routing --
 
-// Thread 0 per job: the union of its palette tiles decides its path -- the
+// A warp per job: the union of its palette tiles decides its path -- the
 // few-values path when it holds at most kShfFastItems values, no accumulator
 // of the reference could overflow and the chunk is within the formulation's
-// column bound, else the general slides.
-__global__ void shf_route(const ShfJob* __restrict__ jobs, const ShfJob single, const uint32_t kcap_h,
+// column bound, else the general slides.  Lane t holds the values of the tiles
+// t, t + 32, ...; the union comes out ascending, one warp minimum per value.
+__global__ void __launch_bounds__(32) shf_route(const ShfJob* __restrict__ jobs, const ShfJob single, const uint32_t kcap_h,
 	const uint32_t dense_max_cols, const uint32_t dense_form) {
 	const ShfJob& J = pick(jobs, single);
-	if (threadIdx.x != 0u) {
-		return;
-	}
+	const uint32_t lane = threadIdx.x;
+	const uint32_t tiles = (J.H + 2u * J.r + kShfPaletteRows - 1u) / kShfPaletteRows;
 	uint32_t vals[kShfFastItems];
 	uint32_t n = 0u;
-	const bool fits = palette_union(J, vals, n);
+	bool fits = true;
+	for (uint32_t t = lane; t < tiles; t += 32u) {
+		fits = fits && J.fast[kSlotWords * (1u + t)] != kNoValue;
+	}
+	fits = __all_sync(0xFFFFFFFFu, fits);
+	uint32_t next = 0u; // the smallest value not yet listed is sought from here
+	while (fits) {
+		uint32_t least = kNoValue;
+		for (uint32_t t = lane; t < tiles; t += 32u) {
+			const uint32_t* const slot = J.fast + kSlotWords * (1u + t);
+			const uint4 w = make_uint4(slot[2], slot[3], slot[4], slot[5]);
+			const uint32_t c = slot[0];
+			const uint32_t words[4] = { w.x, w.y, w.z, w.w };
+#pragma unroll
+			for (uint32_t i = 0u; i < kShfFastItems; i++) {
+				const uint32_t v = (words[i / 2u] >> (16u * (i & 1u))) & 0xFFFFu;
+				least = i < c && v >= next ? min(least, v) : least;
+			}
+		}
+		least = __reduce_min_sync(0xFFFFFFFFu, least);
+		if (least == kNoValue) {
+			break;
+		}
+		if (n == kShfFastItems) {
+			fits = false;
+			break;
+		}
+#pragma unroll
+		for (uint32_t i = 0u; i < kShfFastItems; i++) {
+			vals[i] = i == n ? least : vals[i];
+		}
+		n++;
+		next = least + 1u;
+	}
+	if (lane != 0u) {
+		return;
+	}
 	const uint64_t side = 2ull * J.r + 1u;
 	const uint64_t items = n;
 	const bool radius_ok = J.r <= kFastMaxRadius;
@@ -79,39 +117,54 @@ __global__ void __launch_bounds__(kPaletteBlock) shf_palette(const ShfJob* __res
 		return;
 	}
 	const uint32_t r1 = min(NR, r0 + kShfPaletteRows);
-	__shared__ uint32_t bits[2048];
+	__shared__ __align__(16) uint32_t bits[2048];
 	// distinct values found so far: every bit is counted once, by the thread whose atomicOr set it
 	__shared__ uint32_t seen, fill;
 	__shared__ uint32_t vals[kShfFastItems];
-	for (uint32_t i = threadIdx.x; i < 2048u; i += kPaletteBlock) {
-		bits[i] = 0u;
+	for (uint32_t i = threadIdx.x; i < 512u; i += kPaletteBlock) {
+		reinterpret_cast<uint4*>(bits)[i] = make_uint4(0u, 0u, 0u, 0u);
 	}
 	if (threadIdx.x == 0u) {
 		seen = 0u;
 		fill = 0u;
 	}
 	__syncthreads();
+	// A warp takes rows, a lane every 32nd sample of them, kPaletteAhead loaded
+	// together: biome maps are coherent, so a lane meets a new value rarely and
+	// only then goes to the map in shared memory.
 	const uint16_t* const base = read_region(J);
-	const uint32_t lane = threadIdx.x & 31u;
-	const uint32_t span = (NC + kPaletteBlock - 1u) / kPaletteBlock * kPaletteBlock;
+	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
 	const volatile uint32_t& seen_now = seen;
-	for (uint32_t row = r0; row < r1; row++) {
+	uint32_t last = kNoValue;
+	auto take = [&](const uint32_t v) {
+		if (v != last) {
+			last = v;
+			const uint32_t bit = 1u << (v & 31u);
+			if (!(bits[v >> 5] & bit) && !(atomicOr(&bits[v >> 5], bit) & bit)) {
+				atomicAdd(&seen, 1u);
+			}
+		}
+	};
+	for (uint32_t row = r0 + warp; row < r1; row += kPaletteBlock / 32u) {
 		// a tile past kShfFastItems values sends its job to the general slides: stop reading
-		// (warp-uniform, so every lane of a warp leaves the match below together)
-		if (__any_sync(0xFFFFFFFFu, seen_now > kShfFastItems)) {
+		if (seen_now > kShfFastItems) {
 			break;
 		}
 		const uint16_t* const src = base + static_cast<uint64_t>(row) * J.pitch;
-		for (uint32_t c = threadIdx.x; c < span; c += kPaletteBlock) {
-			const uint32_t v = c < NC ? static_cast<uint32_t>(__ldg(src + c)) : kNoValue;
-			// one lane per distinct value of the warp sets its bit
-			const uint32_t same = __match_any_sync(0xFFFFFFFFu, v);
-			if (v != kNoValue && static_cast<uint32_t>(__ffs(same) - 1) == lane) {
-				const uint32_t bit = 1u << (v & 31u);
-				if (!(bits[v >> 5] & bit) && !(atomicOr(&bits[v >> 5], bit) & bit)) {
-					atomicAdd(&seen, 1u);
-				}
+		uint32_t c = lane;
+		for (; c + 32u * (kPaletteAhead - 1u) < NC; c += 32u * kPaletteAhead) {
+			uint32_t v[kPaletteAhead];
+#pragma unroll
+			for (uint32_t u = 0u; u < kPaletteAhead; u++) {
+				v[u] = __ldg(src + c + 32u * u);
 			}
+#pragma unroll
+			for (uint32_t u = 0u; u < kPaletteAhead; u++) {
+				take(v[u]);
+			}
+		}
+		for (; c < NC; c += 32u) {
+			take(__ldg(src + c));
 		}
 	}
 	__syncthreads();

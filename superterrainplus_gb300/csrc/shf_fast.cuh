@@ -79,46 +79,6 @@ __device__ __forceinline__ uint32_t local_index(const Palette p, const uint32_t 
 		>> 4;
 }
 
-// Union of a job's palette slots, ascending, in vals[0..n) (kNoValue after);
-// false when a tile or the union holds more than kShfFastItems values.
-__device__ __forceinline__ bool palette_union(const ShfJob& J, uint32_t* const vals, uint32_t& n) {
-	const uint32_t NR = J.H + 2u * J.r;
-	const uint32_t tiles = (NR + kShfPaletteRows - 1u) / kShfPaletteRows;
-	n = 0u;
-	bool ok = true;
-	for (uint32_t t = 0u; t < tiles && ok; t++) {
-		const uint32_t* const slot = J.fast + kSlotWords * (1u + t);
-		const uint32_t c = slot[0];
-		if (c == kNoValue) {
-			ok = false;
-			break;
-		}
-		for (uint32_t i = 0u; i < c && ok; i++) {
-			const uint32_t x = (slot[2u + i / 2u] >> (16u * (i & 1u))) & 0xFFFFu;
-			uint32_t p = 0u;
-			while (p < n && vals[p] < x) {
-				p++;
-			}
-			if (p < n && vals[p] == x) {
-				continue;
-			}
-			if (n == kShfFastItems) {
-				ok = false;
-				break;
-			}
-			for (uint32_t m = n; m > p; m--) {
-				vals[m] = vals[m - 1u];
-			}
-			vals[p] = x;
-			n++;
-		}
-	}
-	for (uint32_t j = n; j < kShfFastItems; j++) {
-		vals[j] = kNoValue;
-	}
-	return ok;
-}
-
 // The palette of a job routed to the dense path, from its record.
 __device__ __forceinline__ Palette record_palette(const ShfFastRecord* const rec) {
 	const uint32_t n = rec->count;
