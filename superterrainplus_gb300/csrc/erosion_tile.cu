@@ -177,6 +177,7 @@ __device__ __forceinline__ int2 brush_point(const ErosionJob& J, const uint32_t 
 // Largest magnitude and mean magnitude of a job's map, and its brush.  Bound
 // by reading the map once.
 __global__ void __launch_bounds__(kBinThreads) tile_measure(const TileArgs A) {
+	chain_begin();
 	const ErosionJob& J = job_of(A, blockIdx.y);
 	TileStat& S = A.stat[blockIdx.y];
 	const uint64_t cells = static_cast<uint64_t>(J.dim_x) * J.dim_y;
@@ -315,6 +316,7 @@ __device__ __forceinline__ void file_group(const TileArgs& A, const uint32_t gro
 }
 
 __global__ void __launch_bounds__(kBinThreads) tile_bin(const TileArgs A) {
+	chain_begin();
 	for (uint32_t j = blockIdx.x * kBinThreads + threadIdx.x; j < A.njobs; j += gridDim.x * kBinThreads) {
 		const ErosionJob& J = job_of(A, j);
 		int k;
@@ -329,6 +331,7 @@ __global__ void __launch_bounds__(kBinThreads) tile_bin(const TileArgs A) {
 // of the L2) and sorts its share of the filed droplets by tile; the first
 // block also lists the tiles that hold any.
 __global__ void __launch_bounds__(kScanThreads) tile_scatter(const TileArgs A, const uint32_t phase) {
+	chain_begin();
 	extern __shared__ uint32_t s_base[]; // per tile
 	__shared__ uint32_t s_sum[32], s_bucket[33];
 	TileControl& C = *A.ctl;
@@ -462,6 +465,7 @@ __device__ __noinline__ int32_t deposit_part(int32_t* const c, const int32_t pit
 // the brush in registers, with weight 0 past the brush's last point.
 template<uint32_t Points, bool Mixed>
 __global__ void __launch_bounds__(kTileThreads, 1) tile_erode(const TileArgs A, const TilePhase F) {
+	chain_begin();
 	extern __shared__ int32_t cells[];
 	__shared__ int2 s_brush[kTileThreads / 32u][32];    // cell, amount in units (float bits)
 	__shared__ int32_t s_taken[kTileThreads / 32u][32]; // units each droplet of the warp took
@@ -813,6 +817,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_erode(const TileArgs A, 
 // trip, the brush in one per 32 points, each point taken by a returning add
 // that gives back what the cell lacked.
 __global__ void __launch_bounds__(kFinishThreads) tile_finish(const TileArgs A) {
+	chain_begin();
 	const uint32_t job = blockIdx.y;
 	const uint32_t n = A.nleft[job];
 	if (n == 0u) {
@@ -1113,12 +1118,11 @@ int erosion_tile_launch(const ErosionJob* host_jobs, const ErosionJob* jobs, con
 	STPGB_CUDA_TRY(cudaMemsetAsync(ws, 0, L.zeroed, stream));
 	const uint32_t mblocks = static_cast<uint32_t>(std::min<uint64_t>((max_cells / 4u + kBinThreads - 1u) / kBinThreads,
 		std::max(1u, 8u * sms / njobs)));
-	tile_measure<<<dim3(std::max(1u, mblocks), njobs), kBinThreads, 0, stream>>>(A);
-	STPGB_CUDA_TRY(cudaGetLastError());
+	STPGB_TRY(launch_chained(tile_measure, dim3(std::max(1u, mblocks), njobs), kBinThreads, 0u, stream, A));
 	const uint64_t group = droplets / groups + 1u;
-	tile_bin<<<static_cast<uint32_t>(std::min<uint64_t>(8u * sms, (group + kBinThreads - 1u) / kBinThreads)), kBinThreads,
-		0, stream>>>(A);
-	STPGB_CUDA_TRY(cudaGetLastError());
+	STPGB_TRY(launch_chained(tile_bin,
+		static_cast<uint32_t>(std::min<uint64_t>(8u * sms, (group + kBinThreads - 1u) / kBinThreads)), kBinThreads, 0u, stream,
+		A));
 	const uint32_t sblocks = static_cast<uint32_t>(std::min<uint64_t>(sms, (2u * group + kScanThreads - 1u) / kScanThreads));
 	const size_t smem = static_cast<size_t>(T) * A.pitch * sizeof(int32_t);
 	const uint32_t points = (max_brush + kTileBrushLanes - 1u) / kTileBrushLanes;
@@ -1132,39 +1136,37 @@ int erosion_tile_launch(const ErosionJob* host_jobs, const ErosionJob* jobs, con
 		auto sx = [&](const uint32_t q) { return (q & 3u) == 1u || (q & 3u) == 2u ? half : 0u; };
 		auto sy = [&](const uint32_t q) { return (q & 3u) == 1u || (q & 3u) == 3u ? half : 0u; };
 		const TilePhase F { p, sx(p), sy(p), sx(p + 1u), sy(p + 1u), p + 1u == phases };
-		tile_scatter<<<sblocks, kScanThreads, L.tiles * sizeof(uint32_t), stream>>>(A, p);
-		STPGB_CUDA_TRY(cudaGetLastError());
+		STPGB_TRY(launch_chained(tile_scatter, sblocks, kScanThreads, L.tiles * sizeof(uint32_t), stream, A, p));
 		auto go = [&](auto kernel) {
-			kernel<<<eblocks, kTileThreads, smem, stream>>>(A, F);
+			return launch_chained(kernel, eblocks, kTileThreads, smem, stream, A, F);
 		};
+		int rc = STPGB_OK;
 		switch (mixed ? 8u : points) {
 		case 1u:
-			go(tile_erode<1u, false>);
+			rc = go(tile_erode<1u, false>);
 			break;
 		case 2u:
-			go(tile_erode<2u, false>);
+			rc = go(tile_erode<2u, false>);
 			break;
 		case 3u:
-			go(tile_erode<3u, false>);
+			rc = go(tile_erode<3u, false>);
 			break;
 		case 5u:
-			go(tile_erode<5u, false>);
+			rc = go(tile_erode<5u, false>);
 			break;
 		case 7u:
-			go(tile_erode<7u, false>);
+			rc = go(tile_erode<7u, false>);
 			break;
 		case 8u:
-			go(points <= 5u ? tile_erode<5u, true> : tile_erode<7u, true>);
+			rc = go(points <= 5u ? tile_erode<5u, true> : tile_erode<7u, true>);
 			break;
 		default:
-			go(tile_erode<7u, true>);
+			rc = go(tile_erode<7u, true>);
 			break;
 		}
-		STPGB_CUDA_TRY(cudaGetLastError());
+		STPGB_TRY(rc);
 	}
-	tile_finish<<<dim3(kFinishBlocks, njobs), kFinishThreads, 0, stream>>>(A);
-	STPGB_CUDA_TRY(cudaGetLastError());
-	return STPGB_OK;
+	return launch_chained(tile_finish, dim3(kFinishBlocks, njobs), kFinishThreads, 0u, stream, A);
 }
 
 namespace {

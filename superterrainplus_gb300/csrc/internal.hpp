@@ -45,6 +45,40 @@ enum : unsigned { SETUP_SHF_SMEM = 0u, SETUP_SHF_BAND_SMEM = 1u, SETUP_EROSION_T
 // serialised under a lock, so concurrent first calls from several host threads set up once.
 int once_per_device(unsigned key, int (*setup)());
 
+// Launches `kernel` so that its blocks may be brought to the SMs while the
+// kernel before it in the stream still runs: every block of such a kernel
+// begins with chain_begin(), which waits until all work before it is complete
+// and visible, and lets the next kernel's blocks be brought up in turn.  What
+// is saved is the gap between two kernels of a chain of short ones (one
+// 64^2 chunk's filter, nine launches: 68 -> 54 us).
+template<class... Params, class... Args>
+int launch_chained(void (*kernel)(Params...), const dim3 grid, const dim3 block, const size_t smem,
+	const cudaStream_t stream, Args&&... args) {
+	cudaLaunchAttribute early {};
+	early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	early.val.programmaticStreamSerializationAllowed = 1;
+	cudaLaunchConfig_t config {};
+	config.gridDim = grid;
+	config.blockDim = block;
+	config.dynamicSmemBytes = smem;
+	config.stream = stream;
+	config.attrs = &early;
+	config.numAttrs = 1u;
+	const cudaError_t e = cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+	if (e != cudaSuccess) {
+		cudaGetLastError();
+		return cuda_fail(e, "cudaLaunchKernelEx");
+	}
+	return STPGB_OK;
+}
+
+#ifdef __CUDACC__
+__device__ __forceinline__ void chain_begin() {
+	asm volatile("griddepcontrol.launch_dependents;");
+	asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+#endif
+
 } // namespace stpgb
 
 #define STPGB_CUDA_TRY(expr)                                   \

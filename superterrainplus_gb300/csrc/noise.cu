@@ -25,6 +25,7 @@ template<uint32_t Block>
 __global__ void __launch_bounds__(Block) multibiome_kernel(const NoiseJob* __restrict__ jobs,
 	const NoiseJob single, const stpgb_permutation perm, const stpgb_biome_property* __restrict__ table,
 	const uint32_t biome_count) {
+	chain_begin();
 	__shared__ uint8_t sperm[512];
 	__shared__ float2 gtab[512];
 	simplex::load_tables(perm, sperm, gtab);
@@ -67,19 +68,14 @@ int noise_launch(const NoiseJob* jobs, const NoiseJob& single, uint32_t njobs, u
 	const dim3 grid(static_cast<uint32_t>((max_pixels + b - 1u) / b), njobs);
 	switch (b) {
 	case 128u:
-		multibiome_kernel<128u><<<grid, 128u, 0, stream>>>(jobs, single, perm, table, biome_count);
-		break;
+		return launch_chained(multibiome_kernel<128u>, grid, 128u, 0u, stream, jobs, single, perm, table, biome_count);
 	case 256u:
-		multibiome_kernel<256u><<<grid, 256u, 0, stream>>>(jobs, single, perm, table, biome_count);
-		break;
+		return launch_chained(multibiome_kernel<256u>, grid, 256u, 0u, stream, jobs, single, perm, table, biome_count);
 	case 512u:
-		multibiome_kernel<512u><<<grid, 512u, 0, stream>>>(jobs, single, perm, table, biome_count);
-		break;
+		return launch_chained(multibiome_kernel<512u>, grid, 512u, 0u, stream, jobs, single, perm, table, biome_count);
 	default:
 		return inval("noise_launch: block size must be 128, 256 or 512");
 	}
-	STPGB_CUDA_TRY(cudaGetLastError());
-	return STPGB_OK;
 }
 
 } // namespace stpgb

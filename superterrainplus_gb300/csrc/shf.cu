@@ -71,6 +71,7 @@ constexpr uint32_t kResolved = 0x80000000u;
 // One upward sweep from the window finds every run start.
 __global__ void __launch_bounds__(kVBlock) shf_vertical(const ShfJob* __restrict__ jobs, const ShfJob single,
 	const uint32_t kcap, const uint32_t segs, const uint32_t seg_len) {
+	chain_begin();
 	const ShfJob& J = pick(jobs, single);
 	if (!shf_job_general(J)) {
 		return; // filtered by the few-values path
@@ -277,6 +278,7 @@ __global__ void __launch_bounds__(kVBlock) shf_vertical(const ShfJob* __restrict
 template<bool Write>
 __global__ void __launch_bounds__(kHBlock) shf_horizontal(const ShfJob* __restrict__ jobs, const ShfJob single,
 	const uint32_t kcap_v, const uint32_t kcap, const uint32_t segs, const uint32_t seg_len) {
+	chain_begin();
 	const ShfJob& J = pick(jobs, single);
 	if (!shf_job_general(J)) {
 		return;
@@ -598,6 +600,7 @@ __global__ void __launch_bounds__(kHBlock) shf_horizontal(const ShfJob* __restri
 // the few-values path has one count per row (segs = 1).
 __global__ void __launch_bounds__(kScanBlock) shf_rowscan(const ShfJob* __restrict__ jobs, const ShfJob single,
 	const uint32_t segs_slide) {
+	chain_begin();
 	const ShfJob& J = pick(jobs, single);
 	const uint32_t segs = shf_job_general(J) ? segs_slide : 1u;
 	const uint32_t slots = J.H * segs;
@@ -714,7 +717,7 @@ void shf_bind_workspace(ShfJob& job, unsigned char* ws, const ShfLayout& l) {
 
 int shf_launch(const ShfJob* jobs, const ShfJob& single, uint32_t njobs, uint32_t max_W, uint32_t max_H,
 	uint32_t max_r, uint32_t kcap_v, uint32_t kcap_h, cudaStream_t stream, const uint32_t segments_wanted,
-	const uint32_t path) {
+	const uint32_t path, const bool clear_status) {
 	STPGB_TRY(once_per_device(SETUP_SHF_SMEM, shf_set_smem_attributes));
 	const uint64_t target_threads = uint64_t { current_sm_count() } * kShfThreadsPerSM;
 	// Segments per column / row: enough threads to fill the GPU when few
@@ -744,16 +747,15 @@ int shf_launch(const ShfJob* jobs, const ShfJob& single, uint32_t njobs, uint32_
 	// kShfFastItems values go the few-values path (shf_fast.cu), the others
 	// the sequential slides; each kernel returns at once for jobs of the other.
 	const ShfFastPlan fast = shf_fast_plan(njobs, max_W, max_H, max_r, path);
-	STPGB_TRY(shf_fast_prepare(jobs, single, njobs, max_W, max_H, max_r, kcap_h, fast, stream));
+	STPGB_TRY(shf_fast_prepare(jobs, single, njobs, max_W, max_H, max_r, kcap_h, fast, clear_status,
+		stream));
 	STPGB_TRY(shf_fast_pass(jobs, single, njobs, max_H, fast, false, stream));
-	shf_vertical<<<vgrid, kVBlock, vsmem, stream>>>(jobs, single, kcap_v, segs_v, len_v);
-	STPGB_CUDA_TRY(cudaGetLastError());
-	shf_horizontal<false><<<hgrid, kHBlock, hsmem, stream>>>(jobs, single, kcap_v, kcap_h, segs_h, len_h);
-	STPGB_CUDA_TRY(cudaGetLastError());
-	shf_rowscan<<<dim3(1u, njobs), kScanBlock, 0, stream>>>(jobs, single, segs_h);
-	STPGB_CUDA_TRY(cudaGetLastError());
-	shf_horizontal<true><<<hgrid, kHBlock, hsmem, stream>>>(jobs, single, kcap_v, kcap_h, segs_h, len_h);
-	STPGB_CUDA_TRY(cudaGetLastError());
+	STPGB_TRY(launch_chained(shf_vertical, vgrid, kVBlock, vsmem, stream, jobs, single, kcap_v, segs_v, len_v));
+	STPGB_TRY(launch_chained(shf_horizontal<false>, hgrid, kHBlock, hsmem, stream, jobs, single, kcap_v, kcap_h, segs_h,
+		len_h));
+	STPGB_TRY(launch_chained(shf_rowscan, dim3(1u, njobs), kScanBlock, 0, stream, jobs, single, segs_h));
+	STPGB_TRY(launch_chained(shf_horizontal<true>, hgrid, kHBlock, hsmem, stream, jobs, single, kcap_v, kcap_h, segs_h,
+		len_h));
 	STPGB_TRY(shf_fast_pass(jobs, single, njobs, max_H, fast, true, stream));
 	return STPGB_OK;
 }
@@ -824,7 +826,6 @@ int stpgb_shf_filter(const uint16_t* samplemap, const stpgb_nn_info* nn, uint32_
 		return STPGB_ECAPACITY;
 	}
 	const cudaStream_t s = as_stream(stream);
-	STPGB_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(uint32_t), s));
 	unsigned char* ws = static_cast<unsigned char*>(workspace);
 	ShfJob job;
 	job.samplemap = samplemap;
@@ -840,7 +841,7 @@ int stpgb_shf_filter(const uint16_t* samplemap, const stpgb_nn_info* nn, uint32_
 	job.bins = bins;
 	job.bins_capacity = bins_capacity;
 	job.status = status;
-	return shf_launch(nullptr, job, 1u, W, H, radius, kv, kh, s);
+	return shf_launch(nullptr, job, 1u, W, H, radius, kv, kh, s, 0u, 0u, true);
 }
 
 int stpgb_shf_filter_path(const stpgb_nn_info* nn, uint32_t radius, uint32_t max_items, const void* workspace,

@@ -54,6 +54,7 @@ constexpr int32_t kNoRow = 1 << 30;
 // 0.12 of the 0.20 ms of a 512^2 chunk's filter.
 __global__ void __launch_bounds__(kCarryBlock) shf_band_carry(const ShfJob* __restrict__ jobs, const ShfJob single,
 	const uint32_t band_rows, const uint32_t col_blocks) {
+	chain_begin();
 	const ShfJob& J = pick(jobs, single);
 	const ShfFastRecord* const rec = reinterpret_cast<const ShfFastRecord*>(J.fast);
 	const uint32_t NC = J.W + 2u * J.r;
@@ -262,6 +263,7 @@ __device__ __forceinline__ uint32_t block_exscan_u32(const uint32_t v, uint32_t*
 template<bool Write, uint32_t Cols>
 __global__ void __launch_bounds__(kFastMaxThreads) shf_band_rows(const ShfJob* __restrict__ jobs, const ShfJob single,
 	const uint32_t band_rows, const uint32_t max_cols) {
+	chain_begin();
 	const ShfJob& J = pick(jobs, single);
 	const ShfFastRecord* const rec = reinterpret_cast<const ShfFastRecord*>(J.fast);
 	if (rec->mode != kShfModeFast) {
@@ -473,17 +475,15 @@ int launch_rows(const ShfJob* jobs, const ShfJob& single, const uint32_t njobs, 
 	const dim3 grid(cfg.bands, njobs);
 	switch (cfg.cols_per_thread) {
 	case 1u:
-		shf_band_rows<Write, 1u><<<grid, cfg.threads, cfg.smem, stream>>>(jobs, single, cfg.band_rows, cfg.max_cols);
-		break;
+		return launch_chained(shf_band_rows<Write, 1u>, grid, cfg.threads, cfg.smem, stream, jobs, single, cfg.band_rows,
+			cfg.max_cols);
 	case 2u:
-		shf_band_rows<Write, 2u><<<grid, cfg.threads, cfg.smem, stream>>>(jobs, single, cfg.band_rows, cfg.max_cols);
-		break;
+		return launch_chained(shf_band_rows<Write, 2u>, grid, cfg.threads, cfg.smem, stream, jobs, single, cfg.band_rows,
+			cfg.max_cols);
 	default:
-		shf_band_rows<Write, 4u><<<grid, cfg.threads, cfg.smem, stream>>>(jobs, single, cfg.band_rows, cfg.max_cols);
-		break;
+		return launch_chained(shf_band_rows<Write, 4u>, grid, cfg.threads, cfg.smem, stream, jobs, single, cfg.band_rows,
+			cfg.max_cols);
 	}
-	STPGB_CUDA_TRY(cudaGetLastError());
-	return STPGB_OK;
 }
 
 int band_set_smem_attributes() {
@@ -518,10 +518,8 @@ ShfBandLaunch shf_band_config(const uint32_t njobs, const uint32_t max_W, const 
 int shf_band_carry_launch(const ShfJob* jobs, const ShfJob& single, const uint32_t njobs, const uint32_t max_W,
 	const uint32_t max_r, const ShfBandLaunch& cfg, cudaStream_t stream) {
 	const uint32_t col_blocks = (max_W + 2u * max_r + kCarryBlock - 1u) / kCarryBlock;
-	shf_band_carry<<<dim3(col_blocks * cfg.bands, njobs), kCarryBlock, 0, stream>>>(jobs, single, cfg.band_rows,
-		col_blocks);
-	STPGB_CUDA_TRY(cudaGetLastError());
-	return STPGB_OK;
+	return launch_chained(shf_band_carry, dim3(col_blocks * cfg.bands, njobs), kCarryBlock, 0u, stream, jobs, single,
+		cfg.band_rows, col_blocks);
 }
 
 int shf_band_rows_launch(const ShfJob* jobs, const ShfJob& single, const uint32_t njobs, const ShfBandLaunch& cfg,

@@ -55,6 +55,7 @@ constexpr uint64_t kSlideRowsPerSM = 256u;
 // t, t + 32, ...; the union comes out ascending, one warp minimum per value.
 __global__ void __launch_bounds__(32) shf_route(const ShfJob* __restrict__ jobs, const ShfJob single, const uint32_t kcap_h,
 	const uint32_t dense_max_cols, const uint32_t dense_form) {
+	chain_begin();
 	const ShfJob& J = pick(jobs, single);
 	const uint32_t lane = threadIdx.x;
 	const uint32_t tiles = (J.H + 2u * J.r + kShfPaletteRows - 1u) / kShfPaletteRows;
@@ -109,12 +110,17 @@ __global__ void __launch_bounds__(32) shf_route(const ShfJob* __restrict__ jobs,
 
 // ---------------------------------------------------------------- palette --
 
-__global__ void __launch_bounds__(kPaletteBlock) shf_palette(const ShfJob* __restrict__ jobs, const ShfJob single) {
+__global__ void __launch_bounds__(kPaletteBlock) shf_palette(const ShfJob* __restrict__ jobs, const ShfJob single,
+	const bool clear_status) {
+	chain_begin();
 	const ShfJob& J = pick(jobs, single);
 	const uint32_t NR = J.H + 2u * J.r, NC = J.W + 2u * J.r;
 	const uint32_t r0 = blockIdx.x * kShfPaletteRows;
 	if (r0 >= NR) {
 		return;
+	}
+	if (clear_status && blockIdx.x == 0u && threadIdx.x == 0u) {
+		*J.status = 0u; // the kernels after this one report into it
 	}
 	const uint32_t r1 = min(NR, r0 + kShfPaletteRows);
 	__shared__ __align__(16) uint32_t bits[2048];
@@ -202,6 +208,7 @@ __global__ void __launch_bounds__(kPaletteBlock) shf_palette(const ShfJob* __res
 // kRing samples stay in shared memory, so only the entering sample is read
 // from global memory, kVertAhead rows early.
 __global__ void __launch_bounds__(kVertBlock) shf_vertical_fast(const ShfJob* __restrict__ jobs, const ShfJob single) {
+	chain_begin();
 	const ShfJob& J = pick(jobs, single);
 	const ShfFastRecord* const rec = reinterpret_cast<const ShfFastRecord*>(J.fast);
 	__shared__ uint8_t ring[kRing][kVertBlock];
@@ -270,6 +277,7 @@ __global__ void __launch_bounds__(kVertBlock) shf_vertical_fast(const ShfJob* __
 // pairs as 16-byte stores where the buffers are 16-byte aligned.
 template<bool Write>
 __global__ void __launch_bounds__(kRowBlock) shf_rows_fast(const ShfJob* __restrict__ jobs, const ShfJob single) {
+	chain_begin();
 	const ShfJob& J = pick(jobs, single);
 	if (reinterpret_cast<const ShfFastRecord*>(J.fast)->mode != kShfModeFast) {
 		return;
@@ -468,20 +476,19 @@ ShfFastPlan shf_fast_plan(const uint32_t njobs, const uint32_t max_W, const uint
 }
 
 int shf_fast_prepare(const ShfJob* jobs, const ShfJob& single, const uint32_t njobs, const uint32_t max_W,
-	const uint32_t max_H, const uint32_t max_r, const uint32_t kcap_h, const ShfFastPlan& plan, cudaStream_t stream) {
+	const uint32_t max_H, const uint32_t max_r, const uint32_t kcap_h, const ShfFastPlan& plan,
+	const bool clear_status, cudaStream_t stream) {
 	const uint32_t tiles = (max_H + 2u * max_r + kShfPaletteRows - 1u) / kShfPaletteRows;
-	shf_palette<<<dim3(tiles, njobs), kPaletteBlock, 0, stream>>>(jobs, single);
-	STPGB_CUDA_TRY(cudaGetLastError());
-	shf_route<<<dim3(1u, njobs), 32u, 0, stream>>>(jobs, single, kcap_h, plan.max_cols,
-		plan.bands ? kShfFormBands : kShfFormSlides);
-	STPGB_CUDA_TRY(cudaGetLastError());
+	STPGB_TRY(launch_chained(shf_palette, dim3(tiles, njobs), kPaletteBlock, 0u, stream, jobs, single,
+		clear_status));
+	STPGB_TRY(launch_chained(shf_route, dim3(1u, njobs), 32u, 0u, stream, jobs, single, kcap_h, plan.max_cols,
+		plan.bands ? kShfFormBands : kShfFormSlides));
 	if (plan.bands) {
 		STPGB_TRY(shf_band_carry_launch(jobs, single, njobs, max_W, max_r, plan.band, stream));
 	} else {
 		const uint32_t ncols = max_W + 2u * max_r;
-		shf_vertical_fast<<<dim3((ncols + kVertBlock - 1u) / kVertBlock, njobs), kVertBlock, 0, stream>>>(jobs,
-			single);
-		STPGB_CUDA_TRY(cudaGetLastError());
+		STPGB_TRY(launch_chained(shf_vertical_fast, dim3((ncols + kVertBlock - 1u) / kVertBlock, njobs), kVertBlock, 0u,
+			stream, jobs, single));
 	}
 	return STPGB_OK;
 }
@@ -493,11 +500,10 @@ int shf_fast_pass(const ShfJob* jobs, const ShfJob& single, const uint32_t njobs
 	} else {
 		const dim3 grid((max_H + kRowBlock - 1u) / kRowBlock, njobs);
 		if (write) {
-			shf_rows_fast<true><<<grid, kRowBlock, 0, stream>>>(jobs, single);
+			STPGB_TRY(launch_chained(shf_rows_fast<true>, grid, kRowBlock, 0u, stream, jobs, single));
 		} else {
-			shf_rows_fast<false><<<grid, kRowBlock, 0, stream>>>(jobs, single);
+			STPGB_TRY(launch_chained(shf_rows_fast<false>, grid, kRowBlock, 0u, stream, jobs, single));
 		}
-		STPGB_CUDA_TRY(cudaGetLastError());
 	}
 	return STPGB_OK;
 }
