@@ -1118,9 +1118,9 @@ int erosion_tile_launch(const ErosionJob* host_jobs, const ErosionJob* jobs, con
 	STPGB_CUDA_TRY(cudaMemsetAsync(ws, 0, L.zeroed, stream));
 	const uint32_t mblocks = static_cast<uint32_t>(std::min<uint64_t>((max_cells / 4u + kBinThreads - 1u) / kBinThreads,
 		std::max(1u, 8u * sms / njobs)));
-	STPGB_TRY(launch_chained(tile_measure, dim3(std::max(1u, mblocks), njobs), kBinThreads, 0u, stream, A));
+	STPGB_TRY(launch_chained(true, tile_measure, dim3(std::max(1u, mblocks), njobs), kBinThreads, 0u, stream, A));
 	const uint64_t group = droplets / groups + 1u;
-	STPGB_TRY(launch_chained(tile_bin,
+	STPGB_TRY(launch_chained(true, tile_bin,
 		static_cast<uint32_t>(std::min<uint64_t>(8u * sms, (group + kBinThreads - 1u) / kBinThreads)), kBinThreads, 0u, stream,
 		A));
 	const uint32_t sblocks = static_cast<uint32_t>(std::min<uint64_t>(sms, (2u * group + kScanThreads - 1u) / kScanThreads));
@@ -1136,9 +1136,9 @@ int erosion_tile_launch(const ErosionJob* host_jobs, const ErosionJob* jobs, con
 		auto sx = [&](const uint32_t q) { return (q & 3u) == 1u || (q & 3u) == 2u ? half : 0u; };
 		auto sy = [&](const uint32_t q) { return (q & 3u) == 1u || (q & 3u) == 3u ? half : 0u; };
 		const TilePhase F { p, sx(p), sy(p), sx(p + 1u), sy(p + 1u), p + 1u == phases };
-		STPGB_TRY(launch_chained(tile_scatter, sblocks, kScanThreads, L.tiles * sizeof(uint32_t), stream, A, p));
+		STPGB_TRY(launch_chained(true, tile_scatter, sblocks, kScanThreads, L.tiles * sizeof(uint32_t), stream, A, p));
 		auto go = [&](auto kernel) {
-			return launch_chained(kernel, eblocks, kTileThreads, smem, stream, A, F);
+			return launch_chained(true, kernel, eblocks, kTileThreads, smem, stream, A, F);
 		};
 		int rc = STPGB_OK;
 		switch (mixed ? 8u : points) {
@@ -1166,7 +1166,7 @@ int erosion_tile_launch(const ErosionJob* host_jobs, const ErosionJob* jobs, con
 		}
 		STPGB_TRY(rc);
 	}
-	return launch_chained(tile_finish, dim3(kFinishBlocks, njobs), kFinishThreads, 0u, stream, A);
+	return launch_chained(true, tile_finish, dim3(kFinishBlocks, njobs), kFinishThreads, 0u, stream, A);
 }
 
 namespace {

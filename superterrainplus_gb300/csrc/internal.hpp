@@ -50,9 +50,12 @@ int once_per_device(unsigned key, int (*setup)());
 // begins with chain_begin(), which waits until all work before it is complete
 // and visible, and lets the next kernel's blocks be brought up in turn.  What
 // is saved is the gap between two kernels of a chain of short ones (one
-// 64^2 chunk's filter, nine launches: 68 -> 54 us).
+// 64^2 chunk's filter, nine launches: 68 -> 53 us).  Without `early_up` the
+// launch is an ordinary one: blocks that wait hold their shared memory, and a
+// full launch of many chunks that lives on its L1 pays for that (the packed
+// slides of a 144-chunk batch 1.53 -> 2.7 ms).
 template<class... Params, class... Args>
-int launch_chained(void (*kernel)(Params...), const dim3 grid, const dim3 block, const size_t smem,
+int launch_chained(const bool early_up, void (*kernel)(Params...), const dim3 grid, const dim3 block, const size_t smem,
 	const cudaStream_t stream, Args&&... args) {
 	cudaLaunchAttribute early {};
 	early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -63,7 +66,7 @@ int launch_chained(void (*kernel)(Params...), const dim3 grid, const dim3 block,
 	config.dynamicSmemBytes = smem;
 	config.stream = stream;
 	config.attrs = &early;
-	config.numAttrs = 1u;
+	config.numAttrs = early_up ? 1u : 0u;
 	const cudaError_t e = cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
 	if (e != cudaSuccess) {
 		cudaGetLastError();

@@ -14,49 +14,78 @@
 #include "noise.cuh"
 #include "simplex.cuh"
 
+#include <algorithm>
+
 namespace stpgb {
 
 namespace {
 
 constexpr uint32_t kNoiseBlock = 256u;
 
-// one pixel per thread; the block size (128, 256 or 512) is the batch tuner's choice
-template<uint32_t Block>
-__global__ void __launch_bounds__(Block) multibiome_kernel(const NoiseJob* __restrict__ jobs,
-	const NoiseJob single, const stpgb_permutation perm, const stpgb_biome_property* __restrict__ table,
-	const uint32_t biome_count) {
-	chain_begin();
-	__shared__ uint8_t sperm[512];
-	__shared__ float2 gtab[512];
-	simplex::load_tables(perm, sperm, gtab);
-	__syncthreads();
+// resident blocks of 256 threads per SM (48 registers)
+constexpr uint32_t kNoiseBlocksPerSM = 5u;
+// most strips of pixels a block takes: past a few the tables' share is gone
+constexpr uint32_t kNoiseStrips = 8u;
 
+// One pixel per thread and strip; a block takes the strips blockIdx.x,
+// blockIdx.x + gridDim.x, ... so that building the tables (two lookups per
+// slot, a modulo) is shared by several strips where a launch has them: 144
+// chunks of 512^2 1.57 ms with one strip a block, 1.29 with up to eight.  A
+// strip's offsets are loaded before the tables are waited for, or while the
+// strip before is computed.  The block size (128, 256 or 512) is the batch
+// tuner's choice.  Bound by instruction issue: about 90 per octave of a bin.
+template<uint32_t Block>
+__global__ void __launch_bounds__(Block, kNoiseBlocksPerSM * 256u / Block) multibiome_kernel(
+	const NoiseJob* __restrict__ jobs, const NoiseJob single, const stpgb_permutation perm,
+	const stpgb_biome_property* __restrict__ table, const uint32_t biome_count) {
+	chain_begin();
+	__shared__ simplex::Tables tables;
 	const NoiseJob& J = jobs ? jobs[blockIdx.y] : single;
 	const uint64_t npix = static_cast<uint64_t>(J.W) * J.H;
-	const uint64_t idx = static_cast<uint64_t>(blockIdx.x) * Block + threadIdx.x;
-	if (idx >= npix) {
-		return;
-	}
-	const uint32_t x = static_cast<uint32_t>(idx % J.W), y = static_cast<uint32_t>(idx / J.W);
+	const uint64_t stride = static_cast<uint64_t>(gridDim.x) * Block;
+	uint64_t idx = static_cast<uint64_t>(blockIdx.x) * Block + threadIdx.x;
+	const uint2* const bins = reinterpret_cast<const uint2*>(J.bins);
+	uint32_t b0 = 0u, b1 = 0u;
+	auto load = [&](const uint64_t i) {
+		b0 = b1 = 0u;
+		if (i < npix) {
+			b0 = J.offsets[i];
+			b1 = J.offsets[i + 1u];
+		}
+	};
+	load(idx);
+	simplex::load_tables(perm, tables);
+	__syncthreads();
 	// HalfDimension = vec2(MapSize) / 2 (SuperDemo+/World/Biomes/STPCommonCompiler.cpp:236)
 	const float half_x = static_cast<float>(J.W) / 2.0f, half_y = static_cast<float>(J.H) / 2.0f;
-	const float fx = (1.0f * x - half_x) + J.off_x, fy = (1.0f * y - half_y) + J.off_y;
-
-	float height = 0.0f;
-	const uint32_t b0 = J.offsets[idx], b1 = J.offsets[idx + 1u];
-	for (uint32_t b = b0; b < b1; b++) {
-		const uint2 raw = __ldg(reinterpret_cast<const uint2*>(J.bins) + b);
-		const uint32_t id = raw.x & 0xFFFFu;
-		const float weight = __uint_as_float(raw.y);
-		if (id >= biome_count) {
-			continue;
+	// the first pixel's place by 32-bit divisions (more than 2^32 pixels have no 32-bit offsets
+	// either), the next ones' by the stride's
+	const uint32_t W = J.W, step = gridDim.x * Block, step_y = step / W, step_x = step - step_y * W;
+	uint32_t y = static_cast<uint32_t>(idx) / W, x = static_cast<uint32_t>(idx) - y * W;
+	for (; idx < npix; x += step_x, y += step_y) {
+		if (x >= W) {
+			x -= W;
+			y++;
 		}
-		const stpgb_biome_property p = table[id];
-		const float f = simplex::fractal(sperm, gtab, fx / p.Scale, fy / p.Scale, p.Octave, p.Persistence,
-			p.Lacunarity);
-		height += weight * (f * p.Variation + p.Depth);
+		const float fx = (1.0f * x - half_x) + J.off_x, fy = (1.0f * y - half_y) + J.off_y;
+		const uint32_t begin = b0, end = b1;
+		idx += stride;
+		load(idx);
+		float height = 0.0f;
+		for (uint32_t b = begin; b < end; b++) {
+			const uint2 raw = __ldg(bins + b);
+			const uint32_t id = raw.x & 0xFFFFu;
+			const float weight = __uint_as_float(raw.y);
+			if (id >= biome_count) {
+				continue;
+			}
+			const stpgb_biome_property p = table[id];
+			const float f = simplex::fractal(tables, fx / p.Scale, fy / p.Scale, p.Octave, p.Persistence,
+				p.Lacunarity);
+			height += weight * (f * p.Variation + p.Depth);
+		}
+		J.out[static_cast<uint64_t>(y) * J.pitch + x] = height;
 	}
-	J.out[static_cast<uint64_t>(y) * J.pitch + x] = height;
 }
 
 } // namespace
@@ -65,14 +94,17 @@ int noise_launch(const NoiseJob* jobs, const NoiseJob& single, uint32_t njobs, u
 	const stpgb_permutation& perm, const stpgb_biome_property* table, uint32_t biome_count, cudaStream_t stream,
 	const uint32_t block) {
 	const uint32_t b = block == 0u ? kNoiseBlock : block;
-	const dim3 grid(static_cast<uint32_t>((max_pixels + b - 1u) / b), njobs);
+	const uint64_t strips = (max_pixels + b - 1u) / b;
+	const uint64_t resident = static_cast<uint64_t>(current_sm_count()) * (kNoiseBlocksPerSM * 256u / b);
+	const uint64_t per = std::min<uint64_t>(std::max<uint64_t>(strips * njobs / resident, 1u), kNoiseStrips);
+	const dim3 grid(static_cast<uint32_t>((strips + per - 1u) / per), njobs);
 	switch (b) {
 	case 128u:
-		return launch_chained(multibiome_kernel<128u>, grid, 128u, 0u, stream, jobs, single, perm, table, biome_count);
+		return launch_chained(njobs == 1u, multibiome_kernel<128u>, grid, 128u, 0u, stream, jobs, single, perm, table, biome_count);
 	case 256u:
-		return launch_chained(multibiome_kernel<256u>, grid, 256u, 0u, stream, jobs, single, perm, table, biome_count);
+		return launch_chained(njobs == 1u, multibiome_kernel<256u>, grid, 256u, 0u, stream, jobs, single, perm, table, biome_count);
 	case 512u:
-		return launch_chained(multibiome_kernel<512u>, grid, 512u, 0u, stream, jobs, single, perm, table, biome_count);
+		return launch_chained(njobs == 1u, multibiome_kernel<512u>, grid, 512u, 0u, stream, jobs, single, perm, table, biome_count);
 	default:
 		return inval("noise_launch: block size must be 128, 256 or 512");
 	}

@@ -750,11 +750,11 @@ int shf_launch(const ShfJob* jobs, const ShfJob& single, uint32_t njobs, uint32_
 	STPGB_TRY(shf_fast_prepare(jobs, single, njobs, max_W, max_H, max_r, kcap_h, fast, clear_status,
 		stream));
 	STPGB_TRY(shf_fast_pass(jobs, single, njobs, max_H, fast, false, stream));
-	STPGB_TRY(launch_chained(shf_vertical, vgrid, kVBlock, vsmem, stream, jobs, single, kcap_v, segs_v, len_v));
-	STPGB_TRY(launch_chained(shf_horizontal<false>, hgrid, kHBlock, hsmem, stream, jobs, single, kcap_v, kcap_h, segs_h,
+	STPGB_TRY(launch_chained(fast.bands, shf_vertical, vgrid, kVBlock, vsmem, stream, jobs, single, kcap_v, segs_v, len_v));
+	STPGB_TRY(launch_chained(fast.bands, shf_horizontal<false>, hgrid, kHBlock, hsmem, stream, jobs, single, kcap_v, kcap_h, segs_h,
 		len_h));
-	STPGB_TRY(launch_chained(shf_rowscan, dim3(1u, njobs), kScanBlock, 0, stream, jobs, single, segs_h));
-	STPGB_TRY(launch_chained(shf_horizontal<true>, hgrid, kHBlock, hsmem, stream, jobs, single, kcap_v, kcap_h, segs_h,
+	STPGB_TRY(launch_chained(fast.bands, shf_rowscan, dim3(1u, njobs), kScanBlock, 0, stream, jobs, single, segs_h));
+	STPGB_TRY(launch_chained(fast.bands, shf_horizontal<true>, hgrid, kHBlock, hsmem, stream, jobs, single, kcap_v, kcap_h, segs_h,
 		len_h));
 	STPGB_TRY(shf_fast_pass(jobs, single, njobs, max_H, fast, true, stream));
 	return STPGB_OK;

@@ -475,13 +475,13 @@ int launch_rows(const ShfJob* jobs, const ShfJob& single, const uint32_t njobs, 
 	const dim3 grid(cfg.bands, njobs);
 	switch (cfg.cols_per_thread) {
 	case 1u:
-		return launch_chained(shf_band_rows<Write, 1u>, grid, cfg.threads, cfg.smem, stream, jobs, single, cfg.band_rows,
+		return launch_chained(true, shf_band_rows<Write, 1u>, grid, cfg.threads, cfg.smem, stream, jobs, single, cfg.band_rows,
 			cfg.max_cols);
 	case 2u:
-		return launch_chained(shf_band_rows<Write, 2u>, grid, cfg.threads, cfg.smem, stream, jobs, single, cfg.band_rows,
+		return launch_chained(true, shf_band_rows<Write, 2u>, grid, cfg.threads, cfg.smem, stream, jobs, single, cfg.band_rows,
 			cfg.max_cols);
 	default:
-		return launch_chained(shf_band_rows<Write, 4u>, grid, cfg.threads, cfg.smem, stream, jobs, single, cfg.band_rows,
+		return launch_chained(true, shf_band_rows<Write, 4u>, grid, cfg.threads, cfg.smem, stream, jobs, single, cfg.band_rows,
 			cfg.max_cols);
 	}
 }
@@ -518,7 +518,7 @@ ShfBandLaunch shf_band_config(const uint32_t njobs, const uint32_t max_W, const 
 int shf_band_carry_launch(const ShfJob* jobs, const ShfJob& single, const uint32_t njobs, const uint32_t max_W,
 	const uint32_t max_r, const ShfBandLaunch& cfg, cudaStream_t stream) {
 	const uint32_t col_blocks = (max_W + 2u * max_r + kCarryBlock - 1u) / kCarryBlock;
-	return launch_chained(shf_band_carry, dim3(col_blocks * cfg.bands, njobs), kCarryBlock, 0u, stream, jobs, single,
+	return launch_chained(true, shf_band_carry, dim3(col_blocks * cfg.bands, njobs), kCarryBlock, 0u, stream, jobs, single,
 		cfg.band_rows, col_blocks);
 }
 

@@ -479,15 +479,15 @@ int shf_fast_prepare(const ShfJob* jobs, const ShfJob& single, const uint32_t nj
 	const uint32_t max_H, const uint32_t max_r, const uint32_t kcap_h, const ShfFastPlan& plan,
 	const bool clear_status, cudaStream_t stream) {
 	const uint32_t tiles = (max_H + 2u * max_r + kShfPaletteRows - 1u) / kShfPaletteRows;
-	STPGB_TRY(launch_chained(shf_palette, dim3(tiles, njobs), kPaletteBlock, 0u, stream, jobs, single,
+	STPGB_TRY(launch_chained(plan.bands, shf_palette, dim3(tiles, njobs), kPaletteBlock, 0u, stream, jobs, single,
 		clear_status));
-	STPGB_TRY(launch_chained(shf_route, dim3(1u, njobs), 32u, 0u, stream, jobs, single, kcap_h, plan.max_cols,
+	STPGB_TRY(launch_chained(plan.bands, shf_route, dim3(1u, njobs), 32u, 0u, stream, jobs, single, kcap_h, plan.max_cols,
 		plan.bands ? kShfFormBands : kShfFormSlides));
 	if (plan.bands) {
 		STPGB_TRY(shf_band_carry_launch(jobs, single, njobs, max_W, max_r, plan.band, stream));
 	} else {
 		const uint32_t ncols = max_W + 2u * max_r;
-		STPGB_TRY(launch_chained(shf_vertical_fast, dim3((ncols + kVertBlock - 1u) / kVertBlock, njobs), kVertBlock, 0u,
+		STPGB_TRY(launch_chained(plan.bands, shf_vertical_fast, dim3((ncols + kVertBlock - 1u) / kVertBlock, njobs), kVertBlock, 0u,
 			stream, jobs, single));
 	}
 	return STPGB_OK;
@@ -500,9 +500,9 @@ int shf_fast_pass(const ShfJob* jobs, const ShfJob& single, const uint32_t njobs
 	} else {
 		const dim3 grid((max_H + kRowBlock - 1u) / kRowBlock, njobs);
 		if (write) {
-			STPGB_TRY(launch_chained(shf_rows_fast<true>, grid, kRowBlock, 0u, stream, jobs, single));
+			STPGB_TRY(launch_chained(plan.bands, shf_rows_fast<true>, grid, kRowBlock, 0u, stream, jobs, single));
 		} else {
-			STPGB_TRY(launch_chained(shf_rows_fast<false>, grid, kRowBlock, 0u, stream, jobs, single));
+			STPGB_TRY(launch_chained(plan.bands, shf_rows_fast<false>, grid, kRowBlock, 0u, stream, jobs, single));
 		}
 	}
 	return STPGB_OK;

