@@ -7,11 +7,12 @@
 //
 // The reference merges the neighbour chunks into a pinned host buffer and
 // then copies it to the device (STPNearestNeighbourTextureBuffer.cpp:18-113);
-// here every chunk is copied straight into its place in the merged device
-// buffer with one 2D copy, and back the same way.  The filter runs on the
-// device, so its output never crosses the bus.  Concurrent callers each take
-// a slot (stream + buffers) from a pool, as the reference takes a pooled
-// stream per call (STPHeightfieldGenerator.cpp:152-156).
+// here the chunks are copied straight into their places in the merged device
+// buffer, and back the same way, by one kernel where the GPU reads host
+// memory.  The filter runs on the device, so its output never crosses the bus.
+// Concurrent callers each take a slot (stream + buffers) from a pool, as the
+// reference takes a pooled stream per call (STPHeightfieldGenerator.cpp:152-156).
+#include "host_rects.hpp"
 #include "internal.hpp"
 #include "shf.cuh"
 
@@ -166,35 +167,50 @@ stpgb_nn_info make_nn(const uint32_t map[2], const uint32_t nn[2]) {
 
 // Copies chunk arrays (host) into / out of the merged device buffer
 // (STPNearestNeighbourTextureBuffer.cpp:94-111, chunk i at local
-// coordinate (i % nx, i / nx), STPChunk.cpp:71-73).
+// coordinate (i % nx, i / nx), STPChunk.cpp:71-73): of the merged map, the
+// columns [x0, x1) and rows [y0, y1).  One kernel where the GPU reads host
+// memory itself, else a 2D copy per chunk.
 template<typename T>
-int merge(T* merged, const T* const* chunks, const stpgb_nn_info& nn, cudaStream_t s) {
+int move_chunks(T* merged, T* const* chunks, const stpgb_nn_info& nn, const bool in, const uint32_t x0, const uint32_t y0,
+	const uint32_t x1, const uint32_t y1, cudaStream_t s) {
 	const uint32_t nx = nn.ChunkNearestNeighbour[0], count = nx * nn.ChunkNearestNeighbour[1];
-	const size_t row = static_cast<size_t>(nn.MapSize[0]) * sizeof(T), total_row = row * nx;
+	const uint32_t W = nn.MapSize[0], H = nn.MapSize[1];
+	const size_t row = static_cast<size_t>(W) * sizeof(T), total_row = row * nx;
+	std::vector<HostRect> rects;
 	for (uint32_t i = 0u; i < count; i++) {
 		if (!chunks[i]) {
 			return inval("neighbour chunk pointer is null");
 		}
-		const size_t ox = static_cast<size_t>(i % nx) * nn.MapSize[0], oy = static_cast<size_t>(i / nx) * nn.MapSize[1];
-		T* const dst = merged + oy * nn.TotalMapSize[0] + ox;
-		STPGB_CUDA_TRY(cudaMemcpy2DAsync(dst, total_row, chunks[i], row, row, nn.MapSize[1], cudaMemcpyHostToDevice, s));
+		const uint32_t ox = i % nx * W, oy = i / nx * H;
+		const uint32_t ax = std::max(x0, ox), ay = std::max(y0, oy), bx = std::min(x1, ox + W), by = std::min(y1, oy + H);
+		if (ax >= bx || ay >= by) {
+			continue;
+		}
+		T* const device = merged + static_cast<size_t>(ay) * nn.TotalMapSize[0] + ax;
+		T* const host = chunks[i] + static_cast<size_t>(ay - oy) * W + (ax - ox);
+		const uint32_t bytes = (bx - ax) * static_cast<uint32_t>(sizeof(T));
+		const uint32_t hp = static_cast<uint32_t>(row), dp = static_cast<uint32_t>(total_row);
+		rects.push_back(in ? HostRect { host, device, hp, dp, bytes, by - ay } : HostRect { device, host, dp, hp, bytes, by - ay });
+	}
+	const bool even = std::all_of(chunks, chunks + count, [](const T* p) { return (reinterpret_cast<uintptr_t>(p) & 1u) == 0u; });
+	if (row * H <= 0x7FFFFFFFull && total_row <= 0xFFFFFFFFull && even && host_memory_direct()) {
+		return copy_host_rects(rects.data(), static_cast<uint32_t>(rects.size()), s);
+	}
+	for (const HostRect& r : rects) {
+		STPGB_CUDA_TRY(cudaMemcpy2DAsync(r.dst, in ? total_row : row, r.src, in ? row : total_row, r.width, r.rows,
+			in ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, s));
 	}
 	return STPGB_OK;
 }
 
 template<typename T>
+int merge(T* merged, const T* const* chunks, const stpgb_nn_info& nn, cudaStream_t s) {
+	return move_chunks<T>(merged, const_cast<T* const*>(chunks), nn, true, 0u, 0u, nn.TotalMapSize[0], nn.TotalMapSize[1], s);
+}
+
+template<typename T>
 int unmerge(T* const* chunks, const T* merged, const stpgb_nn_info& nn, cudaStream_t s) {
-	const uint32_t nx = nn.ChunkNearestNeighbour[0], count = nx * nn.ChunkNearestNeighbour[1];
-	const size_t row = static_cast<size_t>(nn.MapSize[0]) * sizeof(T), total_row = row * nx;
-	for (uint32_t i = 0u; i < count; i++) {
-		if (!chunks[i]) {
-			return inval("neighbour chunk pointer is null");
-		}
-		const size_t ox = static_cast<size_t>(i % nx) * nn.MapSize[0], oy = static_cast<size_t>(i / nx) * nn.MapSize[1];
-		const T* const src = merged + oy * nn.TotalMapSize[0] + ox;
-		STPGB_CUDA_TRY(cudaMemcpy2DAsync(chunks[i], row, src, total_row, row, nn.MapSize[1], cudaMemcpyDeviceToHost, s));
-	}
-	return STPGB_OK;
+	return move_chunks<T>(const_cast<T*>(merged), chunks, nn, false, 0u, 0u, nn.TotalMapSize[0], nn.TotalMapSize[1], s);
 }
 
 bool odd_positive(const uint32_t v[2]) {
@@ -406,7 +422,17 @@ int stpgb_generator_generate(stpgb_generator* g, float* heightfield, const uint1
 	auto body = [&]() -> int {
 		STPGB_TRY(slot->biome.alloc(static_cast<size_t>(nn.TotalMapSize[0]) * nn.TotalMapSize[1]));
 		STPGB_TRY(slot->height.alloc(npix));
-		STPGB_TRY(merge<uint16_t>(slot->biome.p, biomemap, nn, s));
+		// the demo plugin reads the chunk and a border of its filter's radius; any other may read it all
+		uint32_t x0 = 0u, y0 = 0u, x1 = nn.TotalMapSize[0], y1 = nn.TotalMapSize[1];
+		if (g->diversity.generate == stpgb_biomefield_generate && g->diversity.user) {
+			const uint32_t r = static_cast<const stpgb_biomefield*>(g->diversity.user)->radius;
+			const uint32_t cx = W * (nn.ChunkNearestNeighbour[0] / 2u), cy = H * (nn.ChunkNearestNeighbour[1] / 2u);
+			x0 = cx - std::min(cx, r);
+			y0 = cy - std::min(cy, r);
+			x1 = std::min<uint64_t>(x1, static_cast<uint64_t>(cx) + W + r);
+			y1 = std::min<uint64_t>(y1, static_cast<uint64_t>(cy) + H + r);
+		}
+		STPGB_TRY(move_chunks<uint16_t>(slot->biome.p, const_cast<uint16_t* const*>(biomemap), nn, true, x0, y0, x1, y1, s));
 		stpgb_diversity_call call {};
 		call.heightmap = slot->height.p;
 		call.biomemap = slot->biome.p;
