@@ -580,9 +580,9 @@ class DeviceOps:
         return offsets, bins, status
 
     def shf_filter_path(self, workspace, map_size, nn, radius, max_items=0):
-        """The path the last shf_filter call with `workspace` took: 0 the general slides, 1 the
-        few-values packed slides, 2 the few-values row bands (at most 8 distinct values in the
-        chunk's read region)."""
+        """The path the last shf_filter call with `workspace` took: 1 the few-values packed slides, 2
+        the few-values row bands (at most 8 distinct values in the chunk's read region), 0 the general
+        slides or the row bands with palettes per panel."""
         info = NNInfo.make(map_size, nn)
         path = C.c_uint32(0)
         check(lib().stpgb_shf_filter_path(C.byref(info), radius, max_items, C.c_void_p(workspace.data_ptr()),

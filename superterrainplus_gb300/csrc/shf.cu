@@ -703,8 +703,7 @@ ShfLayout shf_layout(uint32_t W, uint32_t H, uint32_t r, uint32_t kcap_v) {
 	l.vn = align256(static_cast<size_t>(H) * kcap_v * ncols * sizeof(uint32_t));
 	l.rows = l.vn + align256(static_cast<size_t>(H) * ncols * sizeof(uint16_t));
 	l.fast = l.rows + align256((static_cast<size_t>(H) * kShfMaxSegments + 1u) * sizeof(uint32_t));
-	const size_t tiles = (static_cast<size_t>(H) + 2u * r + kShfPaletteRows - 1u) / kShfPaletteRows;
-	l.total = l.fast + align256((1u + tiles) * sizeof(ShfFastRecord));
+	l.total = l.fast + align256(sizeof(ShfFastRecord));
 	return l;
 }
 
@@ -743,9 +742,9 @@ int shf_launch(const ShfJob* jobs, const ShfJob& single, uint32_t njobs, uint32_
 		+ 12u * kHBlock) * sizeof(uint32_t);
 	const dim3 vgrid(static_cast<uint32_t>((ncols * segs_v + kVBlock - 1u) / kVBlock), njobs);
 	const dim3 hgrid(static_cast<uint32_t>((static_cast<uint64_t>(max_H) * segs_h + kHBlock - 1u) / kHBlock), njobs);
-	// Every job first takes the palette of its read region: at most
-	// kShfFastItems values go the few-values path (shf_fast.cu), the others
-	// the sequential slides; each kernel returns at once for jobs of the other.
+	// Every job first takes the palette of its read region: few values go the
+	// few-values path (shf_fast.cu), the others the sequential slides; each
+	// kernel returns at once for jobs of the other.
 	const ShfFastPlan fast = shf_fast_plan(njobs, max_W, max_H, max_r, path);
 	STPGB_TRY(shf_fast_prepare(jobs, single, njobs, max_W, max_H, max_r, kcap_h, fast, clear_status,
 		stream));

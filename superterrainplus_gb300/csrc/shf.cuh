@@ -26,7 +26,7 @@ struct ShfJob {
 	uint32_t* vbuf;  // [W+2r][kcap_v][H] packed (item << 16 | count), column-major
 	uint16_t* vn;    // [W+2r][H] entries per vertical histogram
 	uint32_t* rows;  // [H*segments+1] bins per (row, segment), then exclusive prefix + total
-	uint32_t* fast;  // [8] path record (ShfFastRecord), then [palette tiles][8] palette slots
+	uint32_t* fast;  // [8] path record (ShfFastRecord)
 	// output
 	uint32_t* offsets;  // [W*H+1]
 	stpgb_bin* bins;
@@ -35,32 +35,41 @@ struct ShfJob {
 };
 
 // The few-values path (shf_fast.cu, shf_band.cu) filters a chunk whose read
-// region holds at most kShfFastItems distinct sample values; other chunks
+// region holds at most kShfFastItems distinct sample values; its row bands also
+// take chunks of more whose panels hold at most kShfWideItems each; the others
 // take the general slides.  Its packed vertical histograms (12 bytes per
-// column and row, or per band) overlay `vbuf`, which that chunk does not
-// otherwise use.
+// column and row, or per band; 24 with a palette per panel) overlay `vbuf`,
+// which that chunk does not otherwise use.
 constexpr uint32_t kShfFastItems = 8u;
-// A job's path: the general slides or the few-values path.
-constexpr uint32_t kShfModeSlide = 0u, kShfModeFast = 1u;
-// Rows of the read region per palette tile.
-constexpr uint32_t kShfPaletteRows = 32u;
-// The row-band formulation keeps a row's tables in shared memory: at most
-// this many columns (W + 2r), bands of at least this many rows.
+// A job's path: the general slides, the few-values path, or the row bands with
+// a palette of up to kShfWideItems values per panel (a chunk of more values of
+// which no panel holds more).
+constexpr uint32_t kShfWideItems = 16u;
+constexpr uint32_t kShfModeSlide = 0u, kShfModeFast = 1u, kShfModeWide = 2u;
+// Widest chunk (W + 2r) that the row bands take with one palette.
 constexpr uint32_t kShfBandMaxCols = 4096u;
-constexpr uint32_t kShfBandMinRows = 4u;
+// Fewest rows of a band, unless the chunk has fewer.
+constexpr uint32_t kShfBandMinRows = 2u;
 
 // Record of the path a job takes, written by the routing kernel: words
-// {mode, distinct values, formulation (kShfForm*, 0 for the general slides),
-// 0, then the values as 8 uint16, ascending}.
+// {mode, distinct values, formulation (kShfForm*, 0 outside the few-values
+// path), 1 where a panel turned out to hold too many values for mode Wide, then
+// the values as 8 uint16, ascending}.
 struct ShfFastRecord {
-	uint32_t mode, count, form, pad;
+	uint32_t mode, count, form, crowded;
 	uint16_t item[kShfFastItems];
 };
 static_assert(sizeof(ShfFastRecord) == 32u, "record is 8 words");
 
+__device__ __forceinline__ uint32_t shf_job_mode(const ShfJob& J) {
+	const volatile ShfFastRecord* const rec = reinterpret_cast<const volatile ShfFastRecord*>(J.fast);
+	const uint32_t mode = rec->mode;
+	return mode == kShfModeWide && rec->crowded != 0u ? kShfModeSlide : mode;
+}
+
 // the general slides' kernels filter only the jobs routed to them
 __device__ __forceinline__ bool shf_job_general(const ShfJob& J) {
-	return reinterpret_cast<const volatile ShfFastRecord*>(J.fast)->mode == kShfModeSlide;
+	return shf_job_mode(J) == kShfModeSlide;
 }
 
 struct ShfLayout {
@@ -92,13 +101,20 @@ int shf_launch(const ShfJob* jobs, const ShfJob& single, uint32_t njobs, uint32_
 // formulations: sequential slides in packed form (a thread per column, then
 // per row) for launches of many chunks, row bands with prefix scans (a block
 // per band of rows) for launches of few.
+// A launch's cut into bands and panels: bands of `rows` rows, the carry's
+// groups of `group` bands, panels of `cols` columns of the read region.
+struct ShfBandShape {
+	uint32_t rows, group, cols;
+};
 struct ShfBandLaunch {
-	uint32_t band_rows, bands, threads, cols_per_thread, max_cols;
+	ShfBandShape shape;
+	uint32_t bands, groups, panels; // of the largest chunk
 	size_t smem;
 };
 struct ShfFastPlan {
 	bool bands;
-	uint32_t max_cols; // widest chunk (W + 2r) the dense path takes; 0: none
+	uint32_t max_cols; // widest chunk (W + 2r) the few-values path takes; 0: none
+	bool wide; // chunks of more values may take the bands with a palette per panel
 	ShfBandLaunch band;
 };
 // stpgb_shf_set_path's choice (0 = by size)
@@ -112,8 +128,8 @@ int shf_fast_pass(const ShfJob* jobs, const ShfJob& single, uint32_t njobs, uint
 	bool write, cudaStream_t stream);
 // the row-band formulation (shf_band.cu)
 ShfBandLaunch shf_band_config(uint32_t njobs, uint32_t max_W, uint32_t max_H, uint32_t max_r);
-int shf_band_carry_launch(const ShfJob* jobs, const ShfJob& single, uint32_t njobs, uint32_t max_W, uint32_t max_r,
-	const ShfBandLaunch& cfg, cudaStream_t stream);
+int shf_band_carry_launch(const ShfJob* jobs, const ShfJob& single, uint32_t njobs, const ShfBandLaunch& cfg,
+	cudaStream_t stream);
 int shf_band_rows_launch(const ShfJob* jobs, const ShfJob& single, uint32_t njobs, const ShfBandLaunch& cfg,
 	bool write, cudaStream_t stream);
 

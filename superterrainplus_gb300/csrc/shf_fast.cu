@@ -13,10 +13,11 @@
 // run as the reference runs them, one thread per column and per row, so the
 // order is the reference's by construction.
 //
-//   shf_palette       block per (32-row tile of the read region, job):
-//                     distinct values through a 65536-bit map in shared
-//                     memory.
-//   shf_route         warp per job: the path (few-values or general).
+//   shf_palette       block per (tile of the read region, job): distinct
+//                     values through a 65536-bit map in shared memory.
+//   shf_route         one block per job: the path (few-values, row bands with
+//                     a palette per panel, or general); further blocks: those
+//                     palettes.
 //   shf_vertical_fast thread per column: slides the column's vertical
 //                     histogram down all rows and writes it to row-major
 //                     planes in the job's vbuf.
@@ -34,8 +35,8 @@ using namespace shfx;
 namespace {
 
 constexpr uint32_t kPaletteBlock = 512u;
-// samples of a row a lane loads together
-constexpr uint32_t kPaletteAhead = 8u;
+// samples of a row a lane loads together: its share of a tile's
+constexpr uint32_t kPaletteAhead = kTileCols / 32u;
 constexpr uint32_t kVertBlock = 64u;
 constexpr uint32_t kRowBlock = 64u;
 // rows of the vertical slide whose samples are loaded ahead of their use
@@ -48,64 +49,155 @@ constexpr uint64_t kSlideRowsPerSM = 256u;
 
 // ---------------------------------------------------------------- routing --
 
-// A warp per job: the union of its palette tiles decides its path -- the
-// few-values path when it holds at most kShfFastItems values, no accumulator
-// of the reference could overflow and the chunk is within the formulation's
-// column bound, else the general slides.  Lane t holds the values of the tiles
-// t, t + 32, ...; the union comes out ascending, one warp minimum per value.
-__global__ void __launch_bounds__(32) shf_route(const ShfJob* __restrict__ jobs, const ShfJob single, const uint32_t kcap_h,
-	const uint32_t dense_max_cols, const uint32_t dense_form) {
-	chain_begin();
-	const ShfJob& J = pick(jobs, single);
-	const uint32_t lane = threadIdx.x;
-	const uint32_t tiles = (J.H + 2u * J.r + kShfPaletteRows - 1u) / kShfPaletteRows;
-	uint32_t vals[kShfFastItems];
-	uint32_t n = 0u;
-	bool fits = true;
-	for (uint32_t t = lane; t < tiles; t += 32u) {
-		fits = fits && J.fast[kSlotWords * (1u + t)] != kNoValue;
-	}
-	fits = __all_sync(0xFFFFFFFFu, fits);
-	uint32_t next = 0u; // the smallest value not yet listed is sought from here
-	while (fits) {
-		uint32_t least = kNoValue;
-		for (uint32_t t = lane; t < tiles; t += 32u) {
-			const uint32_t* const slot = J.fast + kSlotWords * (1u + t);
-			const uint4 w = make_uint4(slot[2], slot[3], slot[4], slot[5]);
-			const uint32_t c = slot[0];
-			const uint32_t words[4] = { w.x, w.y, w.z, w.w };
-#pragma unroll
-			for (uint32_t i = 0u; i < kShfFastItems; i++) {
-				const uint32_t v = (words[i / 2u] >> (16u * (i & 1u))) & 0xFFFFu;
-				least = i < c && v >= next ? min(least, v) : least;
+constexpr uint32_t kRouteBlock = 256u;
+
+// Puts v into the list (kNoValue: free) unless it is there; false: list full.
+__device__ __forceinline__ bool list_value(uint32_t* const list, const uint32_t most, const uint32_t v) {
+	for (uint32_t i = 0u; i < most; i++) {
+		const uint32_t held = const_cast<volatile uint32_t*>(list)[i];
+		if (held == v) {
+			return true;
+		}
+		if (held == kNoValue) {
+			const uint32_t old = atomicCAS(&list[i], kNoValue, v);
+			if (old == kNoValue || old == v) {
+				return true;
 			}
 		}
-		least = __reduce_min_sync(0xFFFFFFFFu, least);
-		if (least == kNoValue) {
-			break;
-		}
-		if (n == kShfFastItems) {
-			fits = false;
-			break;
-		}
-#pragma unroll
-		for (uint32_t i = 0u; i < kShfFastItems; i++) {
-			vals[i] = i == n ? least : vals[i];
-		}
-		n++;
-		next = least + 1u;
 	}
-	if (lane != 0u) {
+	return false;
+}
+
+// The values of the tiles (rows [tr0, tr1), columns [tc0, tc1)) into the list,
+// by thread t of n; false where they or a tile's own are too many.
+__device__ __forceinline__ bool list_tiles(const ShfJob& J, const uint32_t tr0, const uint32_t tr1, const uint32_t tc0,
+	const uint32_t tc1, uint32_t* const list, const uint32_t most, const uint32_t t, const uint32_t n) {
+	const uint32_t across = tc1 - tc0, tiles = (tr1 - tr0) * across, TC = tile_cols(J);
+	uint32_t last = kNoValue;
+	for (uint32_t i = t; i < tiles; i += n) {
+		const uint4* const slot = reinterpret_cast<const uint4*>(tile_slot(J, (tr0 + i / across) * TC + tc0 + i % across));
+		const uint4 a = slot[0], b = slot[1], c = slot[2];
+		const uint32_t held = a.x;
+		if (held > most) {
+			return false;
+		}
+		const uint32_t words[kShfWideItems / 2u] = { a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y };
+#pragma unroll
+		for (uint32_t k = 0u; k < kShfWideItems; k++) {
+			const uint32_t v = (words[k / 2u] >> (16u * (k & 1u))) & 0xFFFFu;
+			if (k < held && v != last) {
+				if (!list_value(list, most, v)) {
+					return false;
+				}
+				last = v;
+			}
+		}
+	}
+	return true;
+}
+
+// Blocks (x, job).  Block 0 decides the job's path from the palette tiles: the
+// few-values path when their union holds at most kShfFastItems values, no
+// accumulator of the reference could overflow and the chunk is within the
+// formulation's column bound; else, in launches of row bands, a palette per
+// panel, as long as none is crowded; else the general slides.  The further
+// blocks, a warp per (group of bands, panel), make those palettes: the values
+// of the rows that the group's windows touch, of the row above them (which the
+// reference's accumulators still hold when they take the window's last) and of
+// the panel's columns.
+__global__ void __launch_bounds__(kRouteBlock) shf_route(const ShfJob* __restrict__ jobs, const ShfJob single,
+	const uint32_t kcap_h, const uint32_t dense_max_cols, const uint32_t dense_form, const bool wide_launch,
+	const ShfBandShape shape) {
+	chain_begin();
+	const ShfJob& J = pick(jobs, single);
+	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+	const uint32_t NC = J.W + 2u * J.r;
+	const uint64_t side = 2ull * J.r + 1u;
+	ShfFastRecord* const rec = reinterpret_cast<ShfFastRecord*>(J.fast);
+	if (!has_palette(J)) {
+		if (blockIdx.x == 0u && threadIdx.x == 0u) {
+			write_record(J, kShfModeSlide, 0u, nullptr, 0u);
+		}
 		return;
 	}
-	const uint64_t side = 2ull * J.r + 1u;
-	const uint64_t items = n;
-	const bool radius_ok = J.r <= kFastMaxRadius;
-	// the packed vertical histograms (12 bytes per column and row, or per band) fit in vbuf
-	// (4 * kcap_v bytes per column and row)
-	const bool dense = fits && radius_ok && J.W + 2u * J.r <= dense_max_cols
-		&& min(items, side + 1u) <= J.kcap_v && min(items, (side + 1u) * side) <= kcap_h && J.kcap_v >= 3u;
-	write_record(J, dense ? kShfModeFast : kShfModeSlide, dense ? n : 0u, vals, dense_form);
+	auto allowed = [&](const uint64_t items) {
+		return min(items, side + 1u) <= J.kcap_v && min(items, (side + 1u) * side) <= kcap_h;
+	};
+	// a launch of bands: its panels' columns (12 bytes per column and band, 24 with a palette per panel) fit in
+	// vbuf, the panels' palettes in vn and the tiles' before them
+	bool columns_fit = J.kcap_v >= 3u, wide = wide_launch;
+	uint32_t groups = 0u, panels = 0u, step = 0u;
+	if (shape.rows != 0u) {
+		const Panels P(J, shape.cols);
+		const uint64_t bands = (J.H + shape.rows - 1u) / shape.rows;
+		panels = P.count;
+		step = P.step;
+		groups = static_cast<uint32_t>((bands + shape.group - 1u) / shape.group);
+		columns_fit = columns_fit && 12ull * bands * P.columns <= vbuf_bytes(J);
+		wide = wide && 24ull * bands * P.columns <= vbuf_bytes(J)
+			&& 4ull * kSlotWords * groups * panels <= vn_bytes(J) && tiles_bytes(J) <= vbuf_bytes(J);
+	}
+	__shared__ uint32_t list[kRouteBlock / 32u][kShfWideItems];
+	for (uint32_t i = threadIdx.x; i < kRouteBlock / 32u * kShfWideItems; i += kRouteBlock) {
+		(&list[0][0])[i] = kNoValue;
+	}
+	__syncthreads();
+	// value `lane` of a full list, in ascending order: by rank
+	auto count_of = [&](const uint32_t* const l) {
+		return static_cast<uint32_t>(__popc(__ballot_sync(0xFFFFFFFFu, lane < kShfWideItems && l[lane] != kNoValue)));
+	};
+	auto rank_of = [&](const uint32_t* const l, const uint32_t v) {
+		uint32_t below = 0u;
+		for (uint32_t i = 0u; i < kShfWideItems; i++) {
+			below += l[i] < v ? 1u : 0u;
+		}
+		return below;
+	};
+	if (blockIdx.x == 0u) {
+		const bool fits = list_tiles(J, 0u, tile_rows(J), 0u, tile_cols(J), list[0], kShfFastItems, threadIdx.x, kRouteBlock);
+		const bool all_fit = __syncthreads_and(fits ? 1 : 0) != 0;
+		__shared__ uint32_t vals[kShfFastItems];
+		if (warp == 0u) {
+			const uint32_t n = count_of(list[0]);
+			if (lane < n) {
+				const uint32_t v = list[0][lane];
+				vals[rank_of(list[0], v)] = v;
+			}
+			__syncwarp();
+			const bool fast = all_fit && allowed(n) && NC <= dense_max_cols && columns_fit;
+			if (lane == 0u) {
+				write_record(J, fast ? kShfModeFast : wide ? kShfModeWide : kShfModeSlide, fast ? n : 0u, vals, dense_form);
+			}
+		}
+		return;
+	}
+	const uint32_t at = (blockIdx.x - 1u) * (kRouteBlock / 32u) + warp;
+	if (!wide || at >= groups * panels) {
+		return;
+	}
+	const uint32_t group = at / panels, panel = at - group * panels;
+	const uint32_t y0 = group * shape.group * shape.rows, y1 = min(J.H, y0 + shape.group * shape.rows);
+	const uint32_t k0 = panel * step, k1 = min(NC, k0 + shape.cols);
+	const bool fits = list_tiles(J, (y0 ? y0 - 1u : 0u) / kTileRows, (y1 - 1u + 2u * J.r) / kTileRows + 1u, k0 / kTileCols,
+		(k1 - 1u) / kTileCols + 1u, list[warp], kShfWideItems, lane, 32u);
+	const bool all_fit = __all_sync(0xFFFFFFFFu, fits);
+	__syncwarp();
+	const uint32_t n = count_of(list[warp]);
+	if (!all_fit || !allowed(n)) {
+		if (lane == 0u) {
+			rec->crowded = 1u;
+		}
+		return;
+	}
+	uint32_t* const pal = panel_slot(J, at);
+	uint16_t* const item = reinterpret_cast<uint16_t*>(pal + 2u);
+	if (lane == 0u) {
+		pal[0] = n;
+	}
+	if (lane < kShfWideItems) {
+		const uint32_t v = list[warp][lane];
+		item[lane < n ? rank_of(list[warp], v) : lane] = static_cast<uint16_t>(v); // 0xFFFF past the count
+	}
 }
 
 // ---------------------------------------------------------------- palette --
@@ -114,86 +206,70 @@ __global__ void __launch_bounds__(kPaletteBlock) shf_palette(const ShfJob* __res
 	const bool clear_status) {
 	chain_begin();
 	const ShfJob& J = pick(jobs, single);
-	const uint32_t NR = J.H + 2u * J.r, NC = J.W + 2u * J.r;
-	const uint32_t r0 = blockIdx.x * kShfPaletteRows;
-	if (r0 >= NR) {
-		return;
-	}
 	if (clear_status && blockIdx.x == 0u && threadIdx.x == 0u) {
 		*J.status = 0u; // the kernels after this one report into it
 	}
-	const uint32_t r1 = min(NR, r0 + kShfPaletteRows);
+	const uint32_t NR = J.H + 2u * J.r, NC = J.W + 2u * J.r;
+	const uint32_t TC = tile_cols(J);
+	if (!has_palette(J) || blockIdx.x >= tile_rows(J) * TC) {
+		return;
+	}
+	if (blockIdx.x == 0u && threadIdx.x == 0u) {
+		reinterpret_cast<ShfFastRecord*>(J.fast)->crowded = 0u;
+	}
+	const uint32_t r0 = blockIdx.x / TC * kTileRows, r1 = min(NR, r0 + kTileRows);
+	const uint32_t c0 = blockIdx.x % TC * kTileCols, c1 = min(NC, c0 + kTileCols);
+	// values met, and the first of them in the order they were met
 	__shared__ __align__(16) uint32_t bits[2048];
-	// distinct values found so far: every bit is counted once, by the thread whose atomicOr set it
-	__shared__ uint32_t seen, fill;
-	__shared__ uint32_t vals[kShfFastItems];
+	__shared__ uint32_t seen, vals[kShfWideItems];
 	for (uint32_t i = threadIdx.x; i < 512u; i += kPaletteBlock) {
 		reinterpret_cast<uint4*>(bits)[i] = make_uint4(0u, 0u, 0u, 0u);
 	}
 	if (threadIdx.x == 0u) {
 		seen = 0u;
-		fill = 0u;
 	}
 	__syncthreads();
-	// A warp takes rows, a lane every 32nd sample of them, kPaletteAhead loaded
-	// together: biome maps are coherent, so a lane meets a new value rarely and
-	// only then goes to the map in shared memory.
+	// A warp takes rows, a lane every 32nd sample of them, all loaded together:
+	// biome maps are coherent, so a lane meets a new value rarely and only then
+	// goes to the map in shared memory.  A value is counted once, by the thread
+	// whose atomicOr set its bit.
 	const uint16_t* const base = read_region(J);
 	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-	const volatile uint32_t& seen_now = seen;
 	uint32_t last = kNoValue;
 	auto take = [&](const uint32_t v) {
-		if (v != last) {
+		if (v != last && v != kNoValue) {
 			last = v;
 			const uint32_t bit = 1u << (v & 31u);
 			if (!(bits[v >> 5] & bit) && !(atomicOr(&bits[v >> 5], bit) & bit)) {
-				atomicAdd(&seen, 1u);
+				const uint32_t i = atomicAdd(&seen, 1u);
+				if (i < kShfWideItems) {
+					vals[i] = v;
+				}
 			}
 		}
 	};
 	for (uint32_t row = r0 + warp; row < r1; row += kPaletteBlock / 32u) {
-		// a tile past kShfFastItems values sends its job to the general slides: stop reading
-		if (seen_now > kShfFastItems) {
-			break;
-		}
 		const uint16_t* const src = base + static_cast<uint64_t>(row) * J.pitch;
-		uint32_t c = lane;
-		for (; c + 32u * (kPaletteAhead - 1u) < NC; c += 32u * kPaletteAhead) {
-			uint32_t v[kPaletteAhead];
+		uint32_t v[kPaletteAhead];
 #pragma unroll
-			for (uint32_t u = 0u; u < kPaletteAhead; u++) {
-				v[u] = __ldg(src + c + 32u * u);
-			}
-#pragma unroll
-			for (uint32_t u = 0u; u < kPaletteAhead; u++) {
-				take(v[u]);
-			}
+		for (uint32_t u = 0u; u < kPaletteAhead; u++) {
+			const uint32_t c = c0 + lane + 32u * u;
+			v[u] = c < c1 ? __ldg(src + c) : kNoValue;
 		}
-		for (; c < NC; c += 32u) {
-			take(__ldg(src + c));
+#pragma unroll
+		for (uint32_t u = 0u; u < kPaletteAhead; u++) {
+			take(v[u]);
 		}
 	}
 	__syncthreads();
-	const uint32_t n = seen;
-	if (n <= kShfFastItems) {
-		for (uint32_t i = threadIdx.x; i < 2048u; i += kPaletteBlock) {
-			uint32_t w = bits[i];
-			while (w) {
-				const uint32_t b = static_cast<uint32_t>(__ffs(w) - 1);
-				w &= w - 1u;
-				vals[atomicAdd(&fill, 1u)] = i * 32u + b;
-			}
+	if (warp == 0u) {
+		uint32_t* const slot = tile_slot(J, blockIdx.x);
+		const uint32_t n = seen;
+		if (lane == 0u) {
+			slot[0] = n <= kShfWideItems ? n : kNoValue;
 		}
-	}
-	__syncthreads();
-	if (threadIdx.x == 0u) {
-		uint32_t* const slot = J.fast + kSlotWords * (1u + blockIdx.x);
-		const bool fits = n <= kShfFastItems;
-		slot[0] = fits ? n : kNoValue;
-		for (uint32_t q = 0u; q < kShfFastItems / 2u; q++) {
-			const uint32_t lo = fits && 2u * q < n ? vals[2u * q] : 0u;
-			const uint32_t hi = fits && 2u * q + 1u < n ? vals[2u * q + 1u] : 0u;
-			slot[2u + q] = lo | (hi << 16);
+		if (lane < min(n, kShfWideItems)) {
+			reinterpret_cast<uint16_t*>(slot + 2u)[lane] = static_cast<uint16_t>(vals[lane]);
 		}
 	}
 }
@@ -469,6 +545,11 @@ ShfFastPlan shf_fast_plan(const uint32_t njobs, const uint32_t max_W, const uint
 	plan.bands = choice == 2u
 		|| (choice == 0u && static_cast<uint64_t>(njobs) * max_H < kSlideRowsPerSM * current_sm_count());
 	plan.max_cols = choice == 3u ? 0u : plan.bands ? kShfBandMaxCols : 0xFFFFFFFFu;
+	// Where the bands run at all, they are the better one for as many values as they take: a 300^2
+	// chunk of 20 biomes 549 us by the general slides, 84 by the bands; 2048^2 of 32 biomes, radius 64,
+	// 1936 and 388; 512^2 of noise of 16 values 19100 and 258.  What a chunk that turns out crowded
+	// pays for the attempt is its panels' palettes, 15-30 us.
+	plan.wide = plan.bands && choice != 3u;
 	if (plan.bands) {
 		plan.band = shf_band_config(njobs, max_W, max_H, max_r);
 	}
@@ -478,13 +559,16 @@ ShfFastPlan shf_fast_plan(const uint32_t njobs, const uint32_t max_W, const uint
 int shf_fast_prepare(const ShfJob* jobs, const ShfJob& single, const uint32_t njobs, const uint32_t max_W,
 	const uint32_t max_H, const uint32_t max_r, const uint32_t kcap_h, const ShfFastPlan& plan,
 	const bool clear_status, cudaStream_t stream) {
-	const uint32_t tiles = (max_H + 2u * max_r + kShfPaletteRows - 1u) / kShfPaletteRows;
+	const uint32_t tiles = ((max_H + 2u * max_r + kTileRows - 1u) / kTileRows)
+		* ((max_W + 2u * max_r + kTileCols - 1u) / kTileCols);
+	const uint32_t palettes = plan.wide ? plan.band.groups * plan.band.panels : 0u;
 	STPGB_TRY(launch_chained(plan.bands, shf_palette, dim3(tiles, njobs), kPaletteBlock, 0u, stream, jobs, single,
 		clear_status));
-	STPGB_TRY(launch_chained(plan.bands, shf_route, dim3(1u, njobs), 32u, 0u, stream, jobs, single, kcap_h, plan.max_cols,
-		plan.bands ? kShfFormBands : kShfFormSlides));
+	STPGB_TRY(launch_chained(plan.bands, shf_route, dim3(1u + (palettes + kRouteBlock / 32u - 1u) / (kRouteBlock / 32u), njobs),
+		kRouteBlock, 0u, stream, jobs, single, kcap_h, plan.max_cols, plan.bands ? kShfFormBands : kShfFormSlides, plan.wide,
+		plan.band.shape));
 	if (plan.bands) {
-		STPGB_TRY(shf_band_carry_launch(jobs, single, njobs, max_W, max_r, plan.band, stream));
+		STPGB_TRY(shf_band_carry_launch(jobs, single, njobs, plan.band, stream));
 	} else {
 		const uint32_t ncols = max_W + 2u * max_r;
 		STPGB_TRY(launch_chained(plan.bands, shf_vertical_fast, dim3((ncols + kVertBlock - 1u) / kVertBlock, njobs), kVertBlock, 0u,

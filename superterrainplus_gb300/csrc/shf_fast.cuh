@@ -18,8 +18,11 @@ namespace stpgb {
 namespace shfx {
 
 constexpr uint32_t kNoValue = 0xFFFFFFFFu;
-// words per palette slot and per record: {count, 0, values as uint16 pairs x4, 0, 0}
-constexpr uint32_t kSlotWords = 8u;
+// words per palette: {count, kNoValue past kShfWideItems; 0; values as uint16 pairs x8; 0, 0}
+constexpr uint32_t kSlotWords = 12u;
+// Rows and columns of the read region per palette tile: a panel's palette is
+// the union of the tiles it touches, so a tile is a fraction of its width.
+constexpr uint32_t kTileRows = 16u, kTileCols = 256u;
 // the byte counts hold 2r+2 (add before remove), the 16-bit fields
 // (2r+1)(2r+2), a column's ring of local indices 2r+2
 constexpr uint32_t kFastMaxRadius = 126u;
@@ -27,6 +30,51 @@ constexpr uint32_t kFastMaxRadius = 126u;
 __device__ __forceinline__ const ShfJob& pick(const ShfJob* jobs, const ShfJob& single) {
 	return jobs ? jobs[blockIdx.y] : single;
 }
+
+__device__ __forceinline__ uint32_t tile_rows(const ShfJob& J) {
+	return (J.H + 2u * J.r + kTileRows - 1u) / kTileRows;
+}
+__device__ __forceinline__ uint32_t tile_cols(const ShfJob& J) {
+	return (J.W + 2u * J.r + kTileCols - 1u) / kTileCols;
+}
+
+// The tiles' palettes lie at the start of the workspace (vbuf, and vn behind
+// it), which every path writes only after the routing has read them.
+__device__ __forceinline__ uint32_t* tile_slot(const ShfJob& J, const uint32_t i) {
+	return J.vbuf + static_cast<size_t>(kSlotWords) * i;
+}
+// the panels' palettes lie in vn, which only the general slides use
+__device__ __forceinline__ uint32_t* panel_slot(const ShfJob& J, const uint32_t i) {
+	return reinterpret_cast<uint32_t*>(J.vn) + static_cast<size_t>(kSlotWords) * i;
+}
+
+__device__ __forceinline__ uint64_t vbuf_bytes(const ShfJob& J) {
+	return 4ull * J.kcap_v * J.H * (J.W + 2u * J.r);
+}
+__device__ __forceinline__ uint64_t vn_bytes(const ShfJob& J) {
+	return 2ull * J.H * (J.W + 2u * J.r);
+}
+__device__ __forceinline__ uint64_t tiles_bytes(const ShfJob& J) {
+	return 4ull * kSlotWords * tile_rows(J) * tile_cols(J);
+}
+// the others go the general slides without a palette
+__device__ __forceinline__ bool has_palette(const ShfJob& J) {
+	return J.r <= kFastMaxRadius && tiles_bytes(J) <= vbuf_bytes(J) + vn_bytes(J);
+}
+
+// A job's panels: panel p covers the columns [p * step, p * step + cols) of the
+// read region and the pixels [p * step + (p ? 1 : 0), p * step + step], so that
+// it also holds the columns of the last window before its first pixel's.
+// (Radius at most kFastMaxRadius and cols above 2r + 1.)
+struct Panels {
+	uint32_t step, count;
+	uint64_t columns; // of all panels: the columns of the read region, 2r+1 more per further panel
+	__device__ __forceinline__ Panels(const ShfJob& J, const uint32_t cols) {
+		step = cols - 2u * J.r - 1u;
+		count = J.W > 1u ? (J.W - 1u + step - 1u) / step : 1u;
+		columns = J.W + 2u * J.r + static_cast<uint64_t>(count - 1u) * (2u * J.r + 1u);
+	}
+};
 
 // first sample of the read region: row sy - r, column sx - r
 __device__ __forceinline__ const uint16_t* read_region(const ShfJob& J) {
@@ -96,8 +144,7 @@ __device__ __forceinline__ void write_record(const ShfJob& J, const uint32_t mod
 	ShfFastRecord* const rec = reinterpret_cast<ShfFastRecord*>(J.fast);
 	rec->mode = mode;
 	rec->count = count;
-	rec->form = mode == kShfModeSlide ? 0u : form;
-	rec->pad = 0u;
+	rec->form = mode == kShfModeFast ? form : 0u;
 	for (uint32_t j = 0u; j < kShfFastItems; j++) {
 		rec->item[j] = static_cast<uint16_t>(j < count ? vals[j] : 0u);
 	}
