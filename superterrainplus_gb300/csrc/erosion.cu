@@ -81,6 +81,20 @@ __device__ __forceinline__ HG height_gradient(const float* __restrict__ map, con
 	return r;
 }
 
+// A one-lane droplet's update, whose old value it does not wait for.  atomicAdd
+// on a float through a generic pointer comes out as an atomic that returns it:
+// the updates answered to their lanes, 16 million sectors on a 128^2 chunk.
+// Droplets of several lanes are no faster without the answers (an 88^2 chunk of
+// brush 2, two lanes, 318 us, with reductions 345).
+template<uint32_t G>
+__device__ __forceinline__ void update(float* const cell, const float v) {
+	if constexpr (G == 1u) {
+		asm volatile("red.global.add.f32 [%0], %1;" ::"l"(__cvta_generic_to_global(cell)), "f"(v) : "memory");
+	} else {
+		atomicAdd(cell, v);
+	}
+}
+
 // Brush points a lane has in flight at once (compare-and-swap mode), and
 // the bound on failed swaps per batch before the plain subtraction.
 constexpr uint32_t kBrushBatch = 8u;
@@ -94,7 +108,10 @@ constexpr uint32_t kCasRetries = 16u;
 // warp as a few coalesced requests instead of one request per point, and a
 // step costs ceil(points / G) read-update round trips instead of one per
 // point.  The eroded amounts are summed over the group with a butterfly,
-// which gives every lane the same total.
+// which gives every lane the same total.  One lane per droplet is bound by the
+// chain of its brush points' reads, one round trip to the L2 each: 2.73 ms on
+// a 500^2 field (150,000 droplets, brush 4, 40 steps) with updates that return
+// the old value, 2.25 without.
 template<uint32_t G, bool ExactClamp>
 __global__ void __launch_bounds__(kErodeBlock) erosion_kernel(const ErosionJob* __restrict__ jobs,
 	const ErosionJob single, const uint32_t* __restrict__ gate) {
@@ -164,7 +181,7 @@ __global__ void __launch_bounds__(kErodeBlock) erosion_kernel(const ErosionJob* 
 				sed -= dep;
 				for (uint32_t c = g; c < 4u; c += G) {
 					const float wx = (c & 1u) ? ox : 1.0f - ox, wy = (c & 2u) ? oy : 1.0f - oy;
-					atomicAdd(map + mi + ((c & 2u) ? pitch : 0u) + (c & 1u), dep * wx * wy);
+					update<G>(map + mi + ((c & 2u) ? pitch : 0u) + (c & 1u), dep * wx * wy);
 				}
 			} else {
 				erode_steps++;
@@ -181,7 +198,7 @@ __global__ void __launch_bounds__(kErodeBlock) erosion_kernel(const ErosionJob* 
 						const float we = ero * bw[p];
 						const float cur = __ldcg(cell);
 						const float ds = fminf(fmaxf(cur, 0.0f), we);
-						atomicAdd(cell, -ds);
+						update<G>(cell, -ds);
 						part += ds;
 						asm volatile("" ::: "memory");
 					}
@@ -234,7 +251,7 @@ __global__ void __launch_bounds__(kErodeBlock) erosion_kernel(const ErosionJob* 
 						for (uint32_t k = 0u; k < kBrushBatch; k++) {
 							if (!done[k]) {
 								const float ds = fminf(fmaxf(cur[k], 0.0f), we[k]);
-								atomicAdd(map + static_cast<int64_t>(mi) + bidx[base + k * G], -ds);
+								update<G>(map + static_cast<int64_t>(mi) + bidx[base + k * G], -ds);
 								part += ds;
 							}
 						}
