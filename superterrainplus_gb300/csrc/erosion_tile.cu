@@ -67,16 +67,20 @@ namespace stpgb {
 
 namespace {
 
-// Threads of an eroding block, one block per SM: 768 (80 registers) took the
-// 4096^2 field's erosion to 41.0 ms, 1024 (64, 72 bytes spilled) to 42.1 with
-// more droplets in flight per tile.
-constexpr uint32_t kTileThreads = 768u;
+// Threads of an eroding block, one block per SM, by the brush points that a
+// lane keeps in registers: 768 (80 registers) took the 4096^2 field's erosion,
+// 9 points, to 36.1 ms, 640 to 36.9 and 512 to 38.8; 14 points spill at 768
+// (1000^2 chunks of radius 6 3.16 ms, at 640 2.93).
+constexpr uint32_t tile_threads(const uint32_t points) {
+	return points <= 9u ? 768u : 640u;
+}
 constexpr uint32_t kTileLeast = 40u, kTileMost = 200u; // sides of a tile
 // A tile's rows lie `side` rounded up to 12 more than a multiple of 32 words
 // apart: rows of the brush up to radius 6 then start in different banks.
 constexpr uint32_t kTilePitchMost = 204u;
-constexpr uint32_t kTileBrushLanes = 16u; // lanes that take one brush
-constexpr uint32_t kTileMostPoints = 7u;  // brush points per lane: up to radius 6
+constexpr uint32_t kTileBrushLanes = 8u;  // lanes that take one brush
+constexpr uint32_t kTileBrushes = 32u / kTileBrushLanes; // brushes a warp takes at a time
+constexpr uint32_t kTileMostPoints = 14u; // brush points per lane: up to radius 6
 constexpr uint32_t kTileMostRadius = 6u;
 constexpr uint32_t kTileMostTiles = 48u * 1024u; // tile_scatter keeps a word of each in shared memory
 constexpr uint32_t kBinThreads = 256u;
@@ -90,8 +94,9 @@ constexpr float kMoveLimit = static_cast<float>(kMoveUnits);
 // adding 1.5 * 2^23 leaves a float's nearest integer in its low bits (|x| < 2^22)
 constexpr float kMagic = 12582912.0f;
 constexpr int32_t kMagicBits = 0x4B400000;
-// lanes without a droplet that make a warp fetch more
-constexpr uint32_t kRefill = 8u;
+// lanes without a droplet that make a warp fetch more (4096^2 field: 2 of them
+// 35.9 ms, 4 35.8, 8 36.1, 12 37.0)
+constexpr uint32_t kRefill = 4u;
 constexpr uint32_t kNoJob = 0xFFFFFFFFu;
 
 struct TileJob {
@@ -460,26 +465,30 @@ __device__ __noinline__ int32_t deposit_part(int32_t* const c, const int32_t pit
 // step is straight-line code for all lanes (those without a droplet, or whose
 // droplet stops, compute on the tile's first cells), since the instructions a
 // step issues bound the kernel, not the shared memory's atomics.  The brushes
-// of a warp's eroding droplets are taken two at a time, 16 lanes each; a lane
+// of a warp's eroding droplets are taken four at a time, 8 lanes each; a lane
 // keeps the tile offsets and the weights of its (at most Points) points of
-// the brush in registers, with weight 0 past the brush's last point.
+// the brush in registers, with weight 0 past the brush's last point, and leaves
+// what it took in shared memory for the droplet's lane to sum.  (Two at a time,
+// 16 lanes each and a warp reduction per pair, spent 1.7 times the instructions
+// on a brush of radius 4 or 5: the 4096^2 field 41.1 ms, now 35.6, the
+// production batch's erosion 18.0 and 15.7.)
 template<uint32_t Points, bool Mixed>
-__global__ void __launch_bounds__(kTileThreads, 1) tile_erode(const TileArgs A, const TilePhase F) {
+__global__ void __launch_bounds__(tile_threads(Points), 1) tile_erode(const TileArgs A, const TilePhase F) {
+	constexpr uint32_t kThreads = tile_threads(Points);
 	chain_begin();
 	extern __shared__ int32_t cells[];
-	__shared__ int2 s_brush[kTileThreads / 32u][32];    // cell, amount in units (float bits)
-	__shared__ int32_t s_taken[kTileThreads / 32u][32]; // units each droplet of the warp took
+	__shared__ int2 s_brush[kThreads / 32u][32];    // cell, amount in units (float bits)
+	__shared__ __align__(16) int32_t s_taken[kThreads / 32u][32u * kTileBrushLanes]; // units each lane took for each
 	__shared__ uint32_t s_work, s_next;
 	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-	const bool upper = lane >= kTileBrushLanes;
 	const uint32_t T = A.T;
 	const int32_t pitch = static_cast<int32_t>(A.pitch);
 	volatile int32_t* const vcells = cells;
 	const uint32_t now = F.phase & 1u, to = now ^ 1u;
 	// the starts of the next phase
 	if (F.phase + 1u < A.groups) {
-		file_group(A, F.phase + 1u, F.next_x, F.next_y, blockIdx.x * kTileThreads + threadIdx.x,
-			gridDim.x * kTileThreads);
+		file_group(A, F.phase + 1u, F.next_x, F.next_y, blockIdx.x * kThreads + threadIdx.x,
+			gridDim.x * kThreads);
 	}
 	const uint32_t nwork = A.ctl->nwork;
 	uint32_t job = kNoJob;
@@ -538,7 +547,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_erode(const TileArgs A, 
 		const int32_t origin = y0 * pitch + x0; // of the tile-local index y * pitch + x
 		const uint32_t width = static_cast<uint32_t>(x1 - x0), area = width * static_cast<uint32_t>(y1 - y0);
 		float* const map = J.map + static_cast<uint64_t>(y0) * J.pitch + x0;
-		for (uint32_t c = threadIdx.x; c < area; c += kTileThreads) {
+		for (uint32_t c = threadIdx.x; c < area; c += kThreads) {
 			const uint32_t y = c / width, x = c - y * width;
 			cells[y * pitch + x] = __float2int_rd(__ldcg(map + static_cast<uint64_t>(y) * J.pitch + x) * scale);
 		}
@@ -675,7 +684,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_erode(const TileArgs A, 
 				}
 				sed -= static_cast<float>(put) * unit;
 			}
-			// the brushes of the warp's eroding droplets, two at a time
+			// the brushes of the warp's eroding droplets, four at a time
 			const bool erode = going && !deposit;
 			const uint32_t emask = __ballot_sync(0xFFFFFFFFu, erode);
 			if (emask != 0u) {
@@ -684,13 +693,14 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_erode(const TileArgs A, 
 				if (erode) {
 					s_brush[warp][mine] = make_int2(cells_at + 4 * at, __float_as_int(amount));
 				}
-				if ((n & 1u) && lane == 0u) {
-					s_brush[warp][n] = make_int2(cells_at + 4 * (R - 1) * (pitch + 1), 0); // nothing for the upper half
+				if (lane < (0u - n) % kTileBrushes) {
+					s_brush[warp][n + lane] = make_int2(cells_at + 4 * (R - 1) * (pitch + 1), 0); // nothing to take
 				}
 				__syncwarp();
-				const int2* mybrush = &s_brush[warp][upper ? 1 : 0];
+				const int2* mybrush = &s_brush[warp][lane / kTileBrushLanes];
+				int32_t* mytaken = &s_taken[warp][lane];
 #pragma unroll 1
-				for (uint32_t b = 0u; b < n; b += 2u, mybrush += 2) {
+				for (uint32_t b = 0u; b < n; b += kTileBrushes, mybrush += kTileBrushes, mytaken += 32) {
 					const int2 B = *mybrush;
 					const float e = __int_as_float(B.y);
 					int32_t bits[Points], old[Points];
@@ -721,15 +731,14 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_erode(const TileArgs A, 
 							}
 						}
 					}
-					const int32_t below = __reduce_add_sync(0xFFFFFFFFu, upper ? 0 : part);
-					const int32_t above = __reduce_add_sync(0xFFFFFFFFu, upper ? part : 0);
-					if (lane == 0u) {
-						*reinterpret_cast<int2*>(&s_taken[warp][b]) = make_int2(below, above);
-					}
+					*mytaken = part;
 				}
 				__syncwarp();
 				if (erode) {
-					sed += static_cast<float>(s_taken[warp][mine]) * unit;
+					// the droplet's eight lanes, two reads apart in the order that leaves no bank twice
+					const int4* const taken = reinterpret_cast<const int4*>(&s_taken[warp][mine * kTileBrushLanes]);
+					const int4 a = taken[(mine >> 2) & 1u], c = taken[((mine >> 2) & 1u) ^ 1u];
+					sed += static_cast<float>(((a.x + a.y) + (a.z + a.w)) + ((c.x + c.y) + (c.z + c.w))) * unit;
 				}
 				__syncwarp();
 			}
@@ -797,7 +806,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_erode(const TileArgs A, 
 		}
 		__syncthreads();
 		// the changed cells, each with its fraction of a unit
-		for (uint32_t c = threadIdx.x; c < area; c += kTileThreads) {
+		for (uint32_t c = threadIdx.x; c < area; c += kThreads) {
 			const uint32_t y = c / width, x = c - y * width;
 			float* const cell = map + static_cast<uint64_t>(y) * J.pitch + x;
 			const float h = __ldcg(cell) * scale;
@@ -960,13 +969,13 @@ int tile_smem_attributes() {
 	const int bytes = static_cast<int>(kTileMost * kTilePitchMost * sizeof(int32_t));
 	STPGB_CUDA_TRY(cudaFuncSetAttribute(tile_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
 		static_cast<int>(kTileMostTiles * sizeof(uint32_t))));
-	STPGB_CUDA_TRY(cudaFuncSetAttribute(tile_erode<1u, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
 	STPGB_CUDA_TRY(cudaFuncSetAttribute(tile_erode<2u, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-	STPGB_CUDA_TRY(cudaFuncSetAttribute(tile_erode<3u, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-	STPGB_CUDA_TRY(cudaFuncSetAttribute(tile_erode<5u, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-	STPGB_CUDA_TRY(cudaFuncSetAttribute(tile_erode<7u, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-	STPGB_CUDA_TRY(cudaFuncSetAttribute(tile_erode<5u, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-	STPGB_CUDA_TRY(cudaFuncSetAttribute(tile_erode<7u, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+	STPGB_CUDA_TRY(cudaFuncSetAttribute(tile_erode<4u, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+	STPGB_CUDA_TRY(cudaFuncSetAttribute(tile_erode<6u, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+	STPGB_CUDA_TRY(cudaFuncSetAttribute(tile_erode<9u, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+	STPGB_CUDA_TRY(cudaFuncSetAttribute(tile_erode<14u, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+	STPGB_CUDA_TRY(cudaFuncSetAttribute(tile_erode<9u, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+	STPGB_CUDA_TRY(cudaFuncSetAttribute(tile_erode<14u, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
 	return STPGB_OK;
 }
 
@@ -1008,12 +1017,14 @@ uint32_t erosion_tile_side(const ErosionJob* jobs, const uint32_t njobs) {
 	return tiles <= kTileMostTiles ? T : 0u;
 }
 
-// Brush points the droplets could erode in all.  Below about 10^9 the phases'
-// launches and their slowest tiles cost more than the L2's atomics: erosion.cu
-// against the tiles at 3x3 chunks, 1 droplet per pixel, brush 5 and 60 steps
-// 1.93 / 2.23 ms at 384^2 (0.6e9 points), 2.81 / 2.39 at 512^2 (1.1e9), 9.90 /
-// 4.43 at 1024^2 (4.3e9); brush 3 and 30 steps 1.48 / 1.78 at 768^2 (0.4e9),
-// 2.84 / 2.20 at 1024^2 (0.8e9), 9.42 / 6.10 at a 2048^2 field (3.1e9).
+// Brush points the droplets could erode in all.  From 10^9 on the tiles are the
+// better by far: erosion.cu against the tiles at 3x3 chunks, 1 droplet per
+// pixel, brush 5 and 60 steps 2.99 / 2.22 ms at 512^2 (1.1e9 points), 9.90 /
+// 4.04 at 1024^2 (4.3e9); 1500^2 field, brush 3, 40 steps 4.29 / 2.47 (1.35e9).
+// Below, the gain shrinks (384^2 1.97 / 1.90 at 0.6e9, 256^2 at 2.2 droplets per
+// pixel 2.21 / 3.40: few tiles hold starts) while small tiles follow the serial
+// order less closely (RMS against the FP64 serial result of 384^2 at 2 droplets
+// per pixel 0.0010 against 0.0005), so those calls keep to erosion.cu.
 bool erosion_tile_pays(const ErosionJob* jobs, const uint32_t njobs) {
 	double points = 0.0;
 	for (uint32_t j = 0u; j < njobs; j++) {
@@ -1137,31 +1148,28 @@ int erosion_tile_launch(const ErosionJob* host_jobs, const ErosionJob* jobs, con
 		auto sy = [&](const uint32_t q) { return (q & 3u) == 1u || (q & 3u) == 3u ? half : 0u; };
 		const TilePhase F { p, sx(p), sy(p), sx(p + 1u), sy(p + 1u), p + 1u == phases };
 		STPGB_TRY(launch_chained(true, tile_scatter, sblocks, kScanThreads, L.tiles * sizeof(uint32_t), stream, A, p));
-		auto go = [&](auto kernel) {
-			return launch_chained(true, kernel, eblocks, kTileThreads, smem, stream, A, F);
+		auto go = [&](auto kernel, const uint32_t most) {
+			return launch_chained(true, kernel, eblocks, tile_threads(most), smem, stream, A, F);
 		};
 		int rc = STPGB_OK;
-		switch (mixed ? 8u : points) {
-		case 1u:
-			rc = go(tile_erode<1u, false>);
-			break;
+		switch (mixed ? 0u : points) {
 		case 2u:
-			rc = go(tile_erode<2u, false>);
+			rc = go(tile_erode<2u, false>, 2u);
 			break;
-		case 3u:
-			rc = go(tile_erode<3u, false>);
+		case 4u:
+			rc = go(tile_erode<4u, false>, 4u);
 			break;
-		case 5u:
-			rc = go(tile_erode<5u, false>);
+		case 6u:
+			rc = go(tile_erode<6u, false>, 6u);
 			break;
-		case 7u:
-			rc = go(tile_erode<7u, false>);
+		case 9u:
+			rc = go(tile_erode<9u, false>, 9u);
 			break;
-		case 8u:
-			rc = go(points <= 5u ? tile_erode<5u, true> : tile_erode<7u, true>);
+		case 14u:
+			rc = go(tile_erode<14u, false>, 14u);
 			break;
 		default:
-			rc = go(tile_erode<7u, true>);
+			rc = points <= 9u ? go(tile_erode<9u, true>, 9u) : go(tile_erode<14u, true>, 14u);
 			break;
 		}
 		STPGB_TRY(rc);
