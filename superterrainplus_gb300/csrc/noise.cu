@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(Block, kNoiseBlocksPerSM * 256u / Block) multi
 				continue;
 			}
 			const stpgb_biome_property p = table[id];
-			const float f = simplex::fractal(tables, fx / p.Scale, fy / p.Scale, p.Octave, p.Persistence,
+			const float f = simplex::fractal<simplex::Rounding::heights>(tables, fx / p.Scale, fy / p.Scale, p.Octave, p.Persistence,
 				p.Lacunarity);
 			height += weight * (f * p.Variation + p.Depth);
 		}

@@ -18,15 +18,20 @@ __device__ __forceinline__ int floori(const float x) {
 	return x > 0.0f ? static_cast<int>(x) : static_cast<int>(x - 1.0f);
 }
 
-// A corner's share from the dot product of its gradient and offset.  Outside
-// its reach the weight is 0 and so is the product: no branch, which the lanes
-// of a warp would take differently.  The roundings are spelled out, here and
-// in the dot products, so that every kernel gets the same noise.
-__device__ __forceinline__ float corner(const float dx, const float dy, const float dot) {
-	float w = fmaxf(__fmaf_rn(-dy, dy, __fmaf_rn(-dx, dx, 0.5f)), 0.0f);
+// A corner's share from its weight before the power, half less its squared
+// distance, and the dot product of its gradient and offset.  Outside its reach
+// the weight is 0 and so is the product: no branch, which the lanes of a warp
+// would take differently.  The roundings are spelled out, here and in the
+// weights and dot products, so that no change of the code around moves a height.
+__device__ __forceinline__ float corner(float w, const float dot) {
+	w = fmaxf(w, 0.0f);
 	w = __fmul_rn(w, w);
 	return __fmul_rn(__fmul_rn(w, w), dot);
 }
+
+// Heights and splatmaps round the squared offset of the middle corner
+// differently, by at most an ulp of the weight; both stay as they are.
+enum class Rounding { heights, splatmap };
 
 // What a block keeps in shared memory for the noise: for every permutation
 // slot j, its value and the next slot's as byte offsets into the gradients
@@ -56,6 +61,7 @@ __device__ __forceinline__ void load_tables(const stpgb_permutation& perm, Table
 // one multiply-add they shift the cell origin by up to an ulp of the sample
 // coordinate, which at world offsets of 10^4-10^5 pixels is a visible error.
 // i + j is added as floats: exact wherever i and j are, below 2^24.
+template<Rounding R>
 __device__ __forceinline__ float simplex2d(const Tables& T, const float x, const float y) {
 	const float s = __fmul_rn(__fadd_rn(x, y), kF2);
 	const int i = floori(__fadd_rn(x, s)), j = floori(__fadd_rn(y, s));
@@ -73,19 +79,21 @@ __device__ __forceinline__ float simplex2d(const Tables& T, const float x, const
 	const float2 g0 = *reinterpret_cast<const float2*>(g + a0);
 	const float2 g1 = *reinterpret_cast<const float2*>(g + (east ? a0 + 8u : a1));
 	const float2 g2 = *reinterpret_cast<const float2*>(g + a1 + 8u);
-	const float c0 = corner(dx0, dy0, __fmaf_rn(g0.y, dy0, __fmul_rn(g0.x, dx0)));
-	const float c1 = corner(dx1, dy1, __fmaf_rn(g1.x, dx1, __fmul_rn(g1.y, dy1)));
-	const float c2 = corner(dx2, dy2, __fmaf_rn(g2.x, dx2, __fmul_rn(g2.y, dy2)));
+	const float x1 = R == Rounding::heights ? __fsub_rn(0.5f, __fmul_rn(dx1, dx1)) : __fmaf_rn(-dx1, dx1, 0.5f);
+	const float c0 = corner(__fmaf_rn(-dy0, dy0, __fmaf_rn(-dx0, dx0, 0.5f)), __fmaf_rn(g0.y, dy0, __fmul_rn(g0.x, dx0)));
+	const float c1 = corner(__fmaf_rn(-dy1, dy1, x1), __fmaf_rn(g1.x, dx1, __fmul_rn(g1.y, dy1)));
+	const float c2 = corner(__fmaf_rn(-dy2, dy2, __fmaf_rn(-dx2, dx2, 0.5f)), __fmaf_rn(g2.x, dx2, __fmul_rn(g2.y, dy2)));
 	return __fmul_rn(70.0f, __fadd_rn(__fadd_rn(c0, c1), c2));
 }
 
 // STPSimplexNoise.cu:84-110 at sample (ux, uy) = ((x - half) + offset) / Scale:
 // the saturated, normalised fractal sum in [0, 1].
+template<Rounding R>
 __device__ __forceinline__ float fractal(const Tables& T, const float ux, const float uy, const uint32_t octave,
 	const float persistence, const float lacunarity) {
 	float sum = 0.0f, amplitude = 1.0f, frequency = 1.0f, range = 0.0f;
 	for (uint32_t o = 0u; o < octave; o++) {
-		sum = __fmaf_rn(simplex2d(T, __fmul_rn(ux, frequency), __fmul_rn(uy, frequency)), amplitude, sum);
+		sum = __fmaf_rn(simplex2d<R>(T, __fmul_rn(ux, frequency), __fmul_rn(uy, frequency)), amplitude, sum);
 		range += amplitude;
 		amplitude *= persistence;
 		frequency *= lacunarity;

@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kSplatTile * kSplatTile) splat_kernel(const cu
 		const float bottom = tex2D<float>(height_tex, fx, fy + kKernelRadius) * kHeightFactor;
 		const float gradient[3] = { top - bottom, kGradientBias, left - right };
 		const float slope = 1.0f - (gradient[1] * rnormf(3, gradient));
-		const float noise = simplex::fractal(tables, noise_x, ((1.0f * y - L.half_y) + C.ChunkMapOffsetY) / kNoiseScale,
+		const float noise = simplex::fractal<simplex::Rounding::splatmap>(tables, noise_x, ((1.0f * y - L.half_y) + C.ChunkMapOffsetY) / kNoiseScale,
 			kNoiseOctaves, kPersistence, kLacunarity) * kNoiseContribution;
 		const uint16_t biome = tex2D<unsigned short>(biome_tex, fx, fy);
 		const float alt = __saturatef(tex2D<float>(height_tex, fx, fy) + noise);
