@@ -790,9 +790,14 @@ int launch_rows(const ShfJob* jobs, const ShfJob& single, const uint32_t njobs, 
 	// a column per thread where a row is one panel (64^2 44 us, with two columns 52; 300^2 of 20 biomes
 	// 84 and 105), two where it is several (1024^2 of 8 biomes 182 us, with two columns 149; 4096^2 of
 	// 32 1.30 ms and 1.20): half the scans per column, and two or three blocks per SM
-	return cfg.panels == 1u
-		? launch_chained(true, shf_band_rows<Write, 1u>, grid, cfg.shape.cols, cfg.smem, stream, jobs, single, cfg.shape)
-		: launch_chained(true, shf_band_rows<Write, 2u>, grid, cfg.shape.cols / 2u, cfg.smem, stream, jobs, single, cfg.shape);
+	const bool one = cfg.panels == 1u;
+	const uint32_t threads = one ? cfg.shape.cols : cfg.shape.cols / 2u;
+	// Blocks that come up while the kernel before still runs pile up on the SMs that it leaves free,
+	// unless an SM holds one of them (64 registers a thread) or they are few: 512^2 82 us, early 76;
+	// 64^2 46 and 44; but 300^2 of 20 biomes 75 and 84, 4096^2 1.16 ms and 1.20.
+	const bool early = threads > 512u || 2ull * cfg.bands * njobs <= current_sm_count();
+	return one ? launch_chained(early, shf_band_rows<Write, 1u>, grid, threads, cfg.smem, stream, jobs, single, cfg.shape)
+			   : launch_chained(early, shf_band_rows<Write, 2u>, grid, threads, cfg.smem, stream, jobs, single, cfg.shape);
 }
 
 uint32_t ceil_div(const uint32_t a, const uint32_t b) {
