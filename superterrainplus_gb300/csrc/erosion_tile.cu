@@ -97,7 +97,7 @@ constexpr int32_t kMagicBits = 0x4B400000;
 // lanes without a droplet that make a warp fetch more (4096^2 field: 2 of them
 // 35.9 ms, 4 35.8, 8 36.1, 12 37.0)
 constexpr uint32_t kRefill = 4u;
-constexpr uint32_t kNoJob = 0xFFFFFFFFu;
+constexpr uint32_t kNoJob = 0xFFFFFFFFu, kNoTile = 0xFFFFFFFFu;
 
 struct TileJob {
 	uint32_t drop0;  // first droplet of the job in the launch's arrays
@@ -120,7 +120,8 @@ struct TileWork {
 
 // zeroed before a launch; what a phase reads was written in the one before, so each comes twice
 struct TileControl {
-	uint32_t filed[2];  // droplets filed for an even / odd phase
+	uint32_t carried[2]; // places of `filed` for the droplets that tiles hand to an even / odd phase
+	uint32_t fresh[2];   // and after them for its starts
 	uint32_t nwork;     // tiles that hold droplets
 	uint32_t cursor[2]; // next tile of the list
 };
@@ -141,7 +142,7 @@ struct TileArgs {
 	TileWork* work;
 	float4* pos;   // x, y, direction
 	float4* flow;  // speed, volume, sediment, steps
-	uint4* filed;  // filed droplets: which, in which tile, at which place there
+	uint4* filed;  // filed droplets: which, in which tile (kNoTile: none), at which place there
 	uint32_t* order; // droplets by tile
 	uint32_t* left;  // per job from its drop0 on: droplets left for tile_finish
 	uint32_t* nleft; // per job
@@ -284,10 +285,15 @@ __device__ __forceinline__ uint32_t group_first(const uint32_t count, const uint
 	return static_cast<uint32_t>(static_cast<uint64_t>(count) * g / groups);
 }
 
-// Files the starts of a group under their tiles, thread `first` of `stride`.
+// Files the starts of a group under their tiles, thread `first` of `stride`,
+// behind the droplets that the tiles hand over.  A start has a place of its own,
+// as a tile's droplets have: places handed out by one counter kept a million
+// droplets of a batch's phase waiting at one address.
 __device__ __forceinline__ void file_group(const TileArgs& A, const uint32_t group, const uint32_t shift_x,
 	const uint32_t shift_y, const uint32_t first, const uint32_t stride) {
-	const uint32_t lane = threadIdx.x & 31u, to = group & 1u;
+	const uint32_t to = group & 1u;
+	uint32_t at = A.ctl->carried[to];
+	uint32_t starts = 0u;
 	for (uint32_t j = 0u; j < A.njobs; j++) {
 		const ErosionJob& J = job_of(A, j);
 		const TileJob& G = geom_of(A, j);
@@ -296,27 +302,22 @@ __device__ __forceinline__ void file_group(const TileArgs& A, const uint32_t gro
 			continue;
 		}
 		const uint32_t d0 = group_first(J.count, A.groups, group), d1 = group_first(J.count, A.groups, group + 1u);
-		for (uint32_t base = d0 + (first - lane); base < d1; base += stride) { // warp-uniform
-			const uint32_t d = base + lane;
-			float px = -1.0f, py = -1.0f;
-			if (d < d1) {
-				px = J.starts[2u * d];
-				py = J.starts[2u * d + 1u];
-			}
+		for (uint32_t d = d0 + first; d < d1; d += stride) {
+			const float px = J.starts[2u * d], py = J.starts[2u * d + 1u];
 			// a start whose 2x2 bilinear footprint is not inside the map dies at once
 			const bool in = px >= 0.0f && px < J.dim_x - 1.0f && py >= 0.0f && py < J.dim_y - 1.0f;
-			const uint32_t mask = __ballot_sync(0xFFFFFFFFu, in);
-			uint32_t at = 0u;
-			if (lane == 0u && mask != 0u) {
-				at = atomicAdd(&A.ctl->filed[to], static_cast<uint32_t>(__popc(mask)));
-			}
-			at = __shfl_sync(0xFFFFFFFFu, at, 0) + static_cast<uint32_t>(__popc(mask & ((1u << lane) - 1u)));
+			uint4 f = make_uint4(0u, kNoTile, 0u, 0u);
 			if (in) {
 				const uint32_t key = tile_at(G, static_cast<uint32_t>(px), static_cast<uint32_t>(py), A.T, shift_x,
 					shift_y);
-				A.filed[at] = make_uint4(G.drop0 + d, key, atomicAdd(A.count[to] + key, 1u), 0u);
+				f = make_uint4(G.drop0 + d, key, atomicAdd(A.count[to] + key, 1u), 0u);
 			}
+			A.filed[at + starts + (d - d0)] = f;
 		}
+		starts += d1 - d0;
+	}
+	if (first == 0u) {
+		A.ctl->fresh[to] = starts;
 	}
 }
 
@@ -338,15 +339,15 @@ __global__ void __launch_bounds__(kBinThreads) tile_bin(const TileArgs A) {
 __global__ void __launch_bounds__(kScanThreads) tile_scatter(const TileArgs A, const uint32_t phase) {
 	chain_begin();
 	extern __shared__ uint32_t s_base[]; // per tile
-	__shared__ uint32_t s_sum[32], s_bucket[33];
+	__shared__ uint32_t s_sum[32], s_bucket[256];
 	TileControl& C = *A.ctl;
 	const uint32_t now = phase & 1u;
 	const uint32_t* const count = A.count[now];
-	const uint32_t n = C.filed[now];
+	const uint32_t n = C.carried[now] + C.fresh[now];
 	const uint32_t per = (A.tiles + kScanThreads - 1u) / kScanThreads;
 	const uint32_t lo = min(A.tiles, threadIdx.x * per), hi = min(A.tiles, lo + per);
 	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-	if (threadIdx.x < 33u) {
+	if (threadIdx.x < 256u) {
 		s_bucket[threadIdx.x] = 0u;
 	}
 	uint32_t sum = 0u;
@@ -383,23 +384,39 @@ __global__ void __launch_bounds__(kScanThreads) tile_scatter(const TileArgs A, c
 		at += count[t];
 	}
 	if (blockIdx.x == 0u) {
-		// the list of the tiles that hold any, those with most droplets first (by powers of two), so
-		// that no block starts on a full tile when the others are done
+		// the list of the tiles that hold any, those with most droplets first (by eighths of powers of
+		// two), so that no block starts on a full tile when the others are done
+		auto bucket = [](const uint32_t c) {
+			const uint32_t z = static_cast<uint32_t>(__clz(c));
+			return 8u * z + 7u - ((c << z) >> 28 & 7u);
+		};
 		for (uint32_t t = lo; t < hi; t++) {
 			const uint32_t c = count[t];
 			if (c != 0u) {
-				atomicAdd(&s_bucket[__clz(c)], 1u);
+				atomicAdd(&s_bucket[bucket(c)], 1u);
 			}
 		}
 		__syncthreads();
-		if (threadIdx.x == 0u) {
-			uint32_t run = 0u;
-			for (uint32_t b = 0u; b < 32u; b++) {
+		if (threadIdx.x < 32u) {
+			uint32_t mine = 0u;
+			for (uint32_t b = 8u * lane; b < 8u * lane + 8u; b++) {
+				mine += s_bucket[b];
+			}
+			uint32_t run = mine;
+#pragma unroll
+			for (uint32_t d = 1u; d < 32u; d <<= 1) {
+				const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, run, d);
+				run += lane >= d ? a : 0u;
+			}
+			if (lane == 31u) {
+				C.nwork = run;
+			}
+			run -= mine;
+			for (uint32_t b = 8u * lane; b < 8u * lane + 8u; b++) {
 				const uint32_t c = s_bucket[b];
 				s_bucket[b] = run;
 				run += c;
 			}
-			C.nwork = run;
 		}
 		__syncthreads();
 		uint32_t job = 0u;
@@ -409,7 +426,7 @@ __global__ void __launch_bounds__(kScanThreads) tile_scatter(const TileArgs A, c
 				while (job + 1u < A.njobs && geom_of(A, job + 1u).tile0 <= t) {
 					job++;
 				}
-				A.work[atomicAdd(&s_bucket[__clz(c)], 1u)] = TileWork { t, s_base[t], c, job };
+				A.work[atomicAdd(&s_bucket[bucket(c)], 1u)] = TileWork { t, s_base[t], c, job };
 			}
 		}
 	}
@@ -418,12 +435,16 @@ __global__ void __launch_bounds__(kScanThreads) tile_scatter(const TileArgs A, c
 		A.count[now ^ 1u][t] = 0u;
 	}
 	if (blockIdx.x == 0u && threadIdx.x == 0u) {
-		C.filed[now ^ 1u] = 0u;
+		C.carried[now ^ 1u] = s_sum[31]; // a place for every droplet of this phase
+		C.fresh[now ^ 1u] = 0u;
 		C.cursor[now] = 0u;
 	}
 	__syncthreads();
 	for (uint32_t i = blockIdx.x * kScanThreads + threadIdx.x; i < n; i += gridDim.x * kScanThreads) {
 		const uint4 f = A.filed[i];
+		if (f.y == kNoTile) {
+			continue;
+		}
 		A.order[s_base[f.y] + f.z] = f.x;
 	}
 }
@@ -479,7 +500,7 @@ __global__ void __launch_bounds__(tile_threads(Points), 1) tile_erode(const Tile
 	extern __shared__ int32_t cells[];
 	__shared__ int2 s_brush[kThreads / 32u][32];    // cell, amount in units (float bits)
 	__shared__ __align__(16) int32_t s_taken[kThreads / 32u][32u * kTileBrushLanes]; // units each lane took for each
-	__shared__ uint32_t s_work, s_next;
+	__shared__ uint32_t s_work, s_next, s_left;
 	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
 	const uint32_t T = A.T;
 	const int32_t pitch = static_cast<int32_t>(A.pitch);
@@ -500,6 +521,7 @@ __global__ void __launch_bounds__(tile_threads(Points), 1) tile_erode(const Tile
 		if (threadIdx.x == 0u) {
 			s_work = atomicAdd(&A.ctl->cursor[now], 1u);
 			s_next = 0u;
+			s_left = 0u;
 		}
 		__syncthreads();
 		const uint32_t wi = s_work;
@@ -766,13 +788,13 @@ __global__ void __launch_bounds__(tile_threads(Points), 1) tile_erode(const Tile
 				const uint32_t out = __ballot_sync(0xFFFFFFFFu, leaves && !F.last);
 				uint32_t from = 0u;
 				if (out != 0u && lane == 0u) {
-					from = atomicAdd(&A.ctl->filed[to], static_cast<uint32_t>(__popc(out)));
+					from = atomicAdd(&s_left, static_cast<uint32_t>(__popc(out)));
 				}
 				from = __shfl_sync(0xFFFFFFFFu, from, 0);
 				if (leaves && !F.last) {
 					const uint32_t key = tile_at(G, static_cast<uint32_t>(px), static_cast<uint32_t>(py), T, F.next_x,
 						F.next_y);
-					A.filed[from + static_cast<uint32_t>(__popc(out & ((1u << lane) - 1u)))] = make_uint4(id, key,
+					A.filed[W.base + from + static_cast<uint32_t>(__popc(out & ((1u << lane) - 1u)))] = make_uint4(id, key,
 						atomicAdd(A.count[to] + key, 1u), 0u);
 				}
 				if (parts) {
@@ -805,6 +827,10 @@ __global__ void __launch_bounds__(tile_threads(Points), 1) tile_erode(const Tile
 			atomicOr(J.status, STATUS_TIMEOUT);
 		}
 		__syncthreads();
+		// the places of the droplets that went no further
+		for (uint32_t i = s_left + threadIdx.x; i < W.count; i += kThreads) {
+			A.filed[W.base + i].y = kNoTile;
+		}
 		// the changed cells, each with its fraction of a unit
 		for (uint32_t c = threadIdx.x; c < area; c += kThreads) {
 			const uint32_t y = c / width, x = c - y * width;
