@@ -84,7 +84,16 @@ def requests(batch, rank):
                  DropletCount=DROPLETS, BrushRadius=BRUSH, Lifetime=LIFETIME) for n in range(batch)]
 
 
-# DRAM bytes and L2 atomic requests of the production batch's erosion launch (16 requests of a 3x3 x
+# DRAM bytes of the production batch's erosion in tiles (16 requests, all its launches) from an ncu
+# capture, and the SM cycles a brush point's returning shared-memory add takes where nothing else runs
+# (9.2 cycles per radius-4 brush of 45 points, brushes at random places of a tile)
+EROSION_TILES_DRAM_BYTES_PER_REQUEST = (1.89e9 + 0.46e9) / 16
+TILE_POINT_CYCLES = 9.2 / 45
+# kernels a batch run launches at most with its erosion on the L2: nine of the filter, noise, four
+# variant groups, format
+L2_KERNELS_PER_RUN = 15
+
+# DRAM bytes and L2 atomic requests of the production batch's erosion launch on the L2 (16 requests of a 3x3 x
 # 512^2 merged map and 600,000 droplets each, all jobs interleaved) from a full ncu capture: 101.04 MB
 # read + 25.90 MB written; 5.106 G atomic requests at the L2 (the brush's returning 16-byte atomics
 # and the scalar deposits) and 0.272 G vector reductions (the deposits whose row pair shares a
@@ -199,6 +208,17 @@ def erosion_l2_roofline(peaks, steps_total, erode_steps, brush_size, stage_ms):
             "frac": t_min / t, "load_bytes": loads, "reduction_bytes": reds,
             "peak_note": "mix-weighted: L2 loads at the measured random 16-byte load rate, reductions at the "
                          "measured random 16-byte vector reduction rate"}
+
+
+def erosion_tile_roofline(erode_steps, brush_size, stage_ms, sms, sm_mhz):
+    """Roofline of the erosion in shared-memory tiles: the brush points its eroding steps take per
+    second against the rate at which the SMs' returning shared-memory adds alone would take them."""
+    points = erode_steps * brush_size
+    achieved = points / (stage_ms / 1000.0) / 1e9
+    peak = sms * sm_mhz * 1e6 / TILE_POINT_CYCLES / 1e9
+    return {"bound": "shared", "achieved": achieved, "peak": peak, "unit": "G brush points/s", "frac": achieved / peak,
+            "brush_points_per_launch": points,
+            "peak_note": "returning shared-memory integer adds of brushes at random places of a tile, measured alone"}
 
 
 def l2_atomic_roofline(peaks, requests, stage_ms):
@@ -545,7 +565,19 @@ def run_ours(args):
     dom = int(np.argmax(stage_ms))
     roof_stage = stage_names[dom]
     roof = None
-    if roof_stage == "hydraulic_erosion":
+    if roof_stage == "hydraulic_erosion" and kernels_per_step > L2_KERNELS_PER_RUN:
+        roof = erosion_tile_roofline(erode_steps, brush_size, stage_ms[dom], peaks["sms"], clocks.summary()["sm_mhz"] or 2070.0)
+        alg_bytes = B * 2 * 9 * S * S * 4
+        roof.update({
+            "kernel": roof_stage, "traffic": EROSION_TILES_DRAM_BYTES_PER_REQUEST * B,
+            "traffic_source": "DRAM read + write of the 16-request production erosion's launches (ncu capture), "
+                              "scaled by the requests per launch",
+            "algorithmic_bytes_per_launch": alg_bytes,
+            "hbm": {"achieved": alg_bytes / (stage_ms[dom] / 1000.0) / 1e9, "peak": peak, "peak_source": peak_kind,
+                    "frac": alg_bytes / (stage_ms[dom] / 1000.0) / 1e9 / peak},
+            "note": "tiles of the map in shared memory; algorithmic bytes: the merged maps read and written once; the "
+                    "instructions of a step bound the kernel before its shared-memory adds do"})
+    elif roof_stage == "hydraulic_erosion":
         roof = erosion_l2_roofline(peaks, steps_total, erode_steps, brush_size, stage_ms[dom])
         alg_bytes = roof["load_bytes"] + roof["reduction_bytes"]
         roof.update({
