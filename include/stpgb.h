@@ -775,7 +775,7 @@ STPGB_API int stpgb_batch_tuning_filter_path(const stpgb_batch* batch, uint32_t*
 
 /* No counterpart in the reference.  The kernels one stpgb_batch_run launches:
  * the kernel nodes of the batch's CUDA graph (the filter's nine launches,
- * noise, one erosion launch per variant group, format). */
+ * noise, one erosion launch per variant group and those of its tiles, format). */
 STPGB_API int stpgb_batch_kernels_per_run(const stpgb_batch* batch, uint32_t* kernels);
 
 /* Realised droplet steps and brush-erosion steps summed over the runs since

@@ -99,6 +99,13 @@ __device__ __forceinline__ void update(float* const cell, const float v) {
 // the bound on failed swaps per batch before the plain subtraction.
 constexpr uint32_t kBrushBatch = 8u;
 constexpr uint32_t kCasRetries = 16u;
+// One-lane droplets: a warp waits for its slowest droplet at every step, so it
+// takes fewer than 32 while the launch has no more than this many warps per SM
+// (half of what is resident, so that all stay in flight): a 64^2 chunk of 9011
+// droplets, 4 per warp, brush 4 and 50 steps, 1.85 -> 1.41 ms; 100^2, 8 per warp, brush 6
+// 5.08 -> 4.88; 128^2, 16 per warp, brush 2 0.52 -> 0.48, brush 3 1.01 -> 1.01.  Beyond that the warps
+// wait for each other instead (128^2, 4 per warp, 1.05).
+constexpr uint32_t kOneLaneWarpsPerSM = 24u;
 
 // G lanes (1, 2, 4, 8, 16 or 32) carry one droplet.  Every lane of a group
 // holds the same droplet state and takes the same branches: the corner
@@ -114,7 +121,7 @@ constexpr uint32_t kCasRetries = 16u;
 // the old value, 2.25 without.
 template<uint32_t G, bool ExactClamp>
 __global__ void __launch_bounds__(kErodeBlock) erosion_kernel(const ErosionJob* __restrict__ jobs,
-	const ErosionJob single, const uint32_t* __restrict__ gate) {
+	const ErosionJob single, const uint32_t* __restrict__ gate, const uint32_t per_warp) {
 	const ErosionJob& J = jobs ? jobs[blockIdx.y] : single;
 	if (gate && gate[blockIdx.y] != 0u) {
 		return; // eroded in tiles
@@ -130,8 +137,8 @@ __global__ void __launch_bounds__(kErodeBlock) erosion_kernel(const ErosionJob* 
 
 	const RainParams& P = J.p;
 	const uint32_t g = threadIdx.x % G;
-	const uint32_t d = (blockIdx.x * kErodeBlock + threadIdx.x) / G;
 	const uint32_t lane = threadIdx.x & 31u;
+	const uint32_t d = lane / G < per_warp ? (blockIdx.x * kErodeBlock + threadIdx.x) / 32u * per_warp + lane / G : J.count;
 	const uint32_t gmask = G == 32u ? 0xFFFFFFFFu : (((1u << G) - 1u) << (lane & ~(G - 1u)));
 	const uint32_t glead = lane & ~(G - 1u);
 	double residual = 0.0;
@@ -1549,7 +1556,14 @@ int erosion_launch(const ErosionJob* jobs, const ErosionJob& single, uint32_t nj
 			return inval("erosion: droplets per group supported with 4, 8 or 16 lanes");
 		}
 	}
-	const uint64_t threads = static_cast<uint64_t>(max_count) * lanes_per_droplet;
+	uint32_t per_warp = 32u / std::max(std::min(lanes_per_droplet, 32u), 1u);
+	if (lanes_per_droplet == 1u && !exact_clamp) {
+		const uint64_t warps = static_cast<uint64_t>(kOneLaneWarpsPerSM) * current_sm_count();
+		while (per_warp > 1u && (max_count + per_warp / 2u - 1u) / (per_warp / 2u) * static_cast<uint64_t>(njobs) <= warps) {
+			per_warp /= 2u;
+		}
+	}
+	const uint64_t threads = (static_cast<uint64_t>(max_count) + per_warp - 1u) / per_warp * 32u;
 	if (threads > 0xFFFFFFFFull - kErodeBlock) {
 		return inval("erosion: too many droplets for one launch");
 	}
@@ -1558,7 +1572,7 @@ int erosion_launch(const ErosionJob* jobs, const ErosionJob& single, uint32_t nj
 		if (smem > 48u * 1024u) {
 			STPGB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
 		}
-		kernel<<<grid, kErodeBlock, smem, stream>>>(jobs, single, gate);
+		kernel<<<grid, kErodeBlock, smem, stream>>>(jobs, single, gate, per_warp);
 		STPGB_CUDA_TRY(cudaGetLastError());
 		return STPGB_OK;
 	};
