@@ -597,11 +597,14 @@ __global__ void __launch_bounds__(kHBlock) shf_horizontal(const ShfJob* __restri
 
 // One block per job: rows[0..H*segs) (row-major over row, segment) ->
 // exclusive prefix, rows[H*segs] = total; offsets[W*H] = total.  A job of
-// the few-values path has one count per row (segs = 1).
+// the packed slides has one count per row (segs = 1).
 __global__ void __launch_bounds__(kScanBlock) shf_rowscan(const ShfJob* __restrict__ jobs, const ShfJob single,
-	const uint32_t segs_slide) {
+	const uint32_t segs_slide, const bool bands) {
 	chain_begin();
 	const ShfJob& J = pick(jobs, single);
+	if (bands && !shf_job_general(J)) {
+		return; // the row bands add their counts up themselves
+	}
 	const uint32_t segs = shf_job_general(J) ? segs_slide : 1u;
 	const uint32_t slots = J.H * segs;
 	__shared__ uint64_t warp_sum[kScanBlock / 32u];
@@ -752,7 +755,7 @@ int shf_launch(const ShfJob* jobs, const ShfJob& single, uint32_t njobs, uint32_
 	STPGB_TRY(launch_chained(fast.bands, shf_vertical, vgrid, kVBlock, vsmem, stream, jobs, single, kcap_v, segs_v, len_v));
 	STPGB_TRY(launch_chained(fast.bands, shf_horizontal<false>, hgrid, kHBlock, hsmem, stream, jobs, single, kcap_v, kcap_h, segs_h,
 		len_h));
-	STPGB_TRY(launch_chained(fast.bands, shf_rowscan, dim3(1u, njobs), kScanBlock, 0, stream, jobs, single, segs_h));
+	STPGB_TRY(launch_chained(fast.bands, shf_rowscan, dim3(1u, njobs), kScanBlock, 0, stream, jobs, single, segs_h, fast.bands));
 	STPGB_TRY(launch_chained(fast.bands, shf_horizontal<true>, hgrid, kHBlock, hsmem, stream, jobs, single, kcap_v, kcap_h, segs_h,
 		len_h));
 	STPGB_TRY(shf_fast_pass(jobs, single, njobs, max_H, fast, true, stream));
