@@ -353,14 +353,18 @@ STPGB_API int stpgb_hydraulic_erosion(float* heightmap, const stpgb_nn_info* nn,
  * STPGB_EROSION_POINTWISE keeps the point-by-point kernels.
  * STPGB_EROSION_EXACT_CLAMP erodes each point by compare-and-swap instead, so
  * racing droplets never remove more than a cell holds (closer to the serial
- * algorithm, slower).  Where the droplets could erode 10^9 brush points or
- * more, the default (lanes_per_droplet = 0, one droplet per group, no flag)
- * erodes the map in tiles held in shared memory instead, with up to 64 MiB of
- * device memory kept between such calls (more is given back); it does so for
- * any size with STPGB_EROSION_TILES.  A call on a stream that is being
- * captured, a map with values that are not finite or a largest magnitude above
- * 64 times the mean one, a brush radius above 6 and lifetimes above 1024 steps
- * keep to the kernels above.  No counterpart in the reference. */
+ * algorithm, slower).  Large calls on wide start areas (10^9 brush points and
+ * 2^20 pixels or more, brushes of 3 and less 2^21, of 30 steps or more) erode
+ * by default (lanes_per_droplet = 0, one droplet per group, no flag) in tiles
+ * of the map held in shared memory instead; any call does so with
+ * STPGB_EROSION_TILES, which explicit lanes or droplets per group and the other
+ * flags override.  The tiles take 56 bytes of device memory per droplet for the
+ * call, of which up to 64 MiB stay between such calls (more is given back);
+ * where it cannot be had, on a stream that is being captured, for a map with
+ * values that are not finite or a largest magnitude above 8 times the mean one,
+ * a brush radius above 6 or more than 1024 steps, the call keeps to the kernels
+ * above, whose results differ from the tiles' as two runs of either do.  No
+ * counterpart in the reference. */
 enum { STPGB_EROSION_EXACT_CLAMP = 1, STPGB_EROSION_POINTWISE = 2, STPGB_EROSION_TILES = 4 };
 
 /* The kernel variant the default (lanes_per_droplet = 0) of

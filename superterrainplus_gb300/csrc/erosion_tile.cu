@@ -23,36 +23,39 @@
 // the last phase through the map in global memory.
 //
 // Droplets race as in the kernels of erosion.cu, and their order matters as
-// much: the starts enter in index order, a group of them a phase, and a tile
-// alternates fresh droplets with those that came from other tiles.  Measured
-// on a production chunk (3x3 x 512^2, 600,000 droplets), RMS against the FP64
-// serial result: 0.0023 with all starts in one phase, 0.0013 in 8 groups,
-// 0.0006 for the kernels of erosion.cu; on a 128^2 chunk at the same density
-// 0.0010 in 8 groups against 0.0025.
+// much: the starts enter in index order, a small group of them a phase (tile_plan),
+// in tiles that a droplet crosses in few phases, and a tile alternates fresh
+// droplets with those that came from other tiles.  With groups of 0.4 droplets
+// per pixel and tiles that put every SM to work the RMS against the FP64 serial
+// result was 1.1 to 2.2 times that of the kernels of erosion.cu; it is 0.67 to
+// 1.05 times theirs.  (Most of either is not the races': a serial run in 32 bits
+// is as far from the one in 64, 0.00117 on a 2048^2 field where the kernels of
+// erosion.cu are at 0.00119 and the tiles at 0.00123.)
 //
 // Inside a tile a height is a 32-bit integer, h * 2^k with 2^k such that the
-// map's largest magnitude lies in [2^25, 2^26): shared memory adds integers
+// map's largest magnitude lies in [2^26, 2^27): shared memory adds integers
 // natively, floats only by compare-and-swap (measured for radius-4 brushes at
 // random places of a 48^2 tile, 1024 threads per SM: 9.2 SM cycles per brush
 // with returning integer adds, 15.3 with returning float adds, 18.6 with
 // compare-and-swap; 9.2, 29.9 and 38.1 when all brushes meet in a 12^2 area).
-// The unit is finer than the spacing of the floats from an eighth of the
-// map's largest height up; amounts are rounded to the nearest unit, sums of
-// units are exact, and a cell's fraction below a unit is kept and added back
-// when the tile is written.  Differences of heights are taken in units, exactly.
+// The unit is no coarser than the spacing of the floats from an eighth of the
+// map's largest height up, where the mean height lies (tile_measure); amounts
+// are rounded to the nearest unit, sums of units are exact, and a cell's
+// fraction below a unit is kept and added back when the tile is written.
+// Differences of heights are taken in units, exactly.
 // A brush point takes its amount w with one returning add and gives back what
 // the cell lacked, so a droplet removes min(max(cell, 0), w) of the cell's
 // exact current value (STPRainDrop.cu:146-157) whoever races it.
 //
 // No sum leaves 32 bits: nothing is put on a cell that was seen at kCellLimit
-// (2^29 units, eight times the map's largest height) or above, no more than
-// kMoveLimit (2^20) at a time, and a block holds at most 768 droplets, so a
-// cell stays below 2^29 + 768 * 2^20 < 2^31.  A droplet that meets a cell at
+// (2^29 units, at least four times the map's largest height) or above, no more
+// than kMoveLimit (2^21) at a time, and a block holds at most 768 droplets, so a
+// cell stays below 2^29 + 768 * 2^21 = 2^31.  A droplet that meets a cell at
 // the limit goes to tile_finish.
 //
 // Maps this arithmetic does not suit (a value that is not finite, a largest
-// magnitude above 64 times the mean one, so that the unit would be coarse for
-// most of the map) and brushes that reach further than their radius are left
+// magnitude above 8 times the mean one, so that the unit would be coarser than
+// the floats of most of the map) and brushes that reach further than their radius are left
 // to the kernels of erosion.cu: tile_measure finds that out per job, and those
 // kernels, launched after, return at once for the jobs eroded here.
 #include "erosion.cuh"
@@ -74,7 +77,7 @@ namespace {
 constexpr uint32_t tile_threads(const uint32_t points) {
 	return points <= 9u ? 768u : 640u;
 }
-constexpr uint32_t kTileLeast = 40u, kTileMost = 200u; // sides of a tile
+constexpr uint32_t kTileLeast = 128u, kTileMost = 200u; // sides of a tile
 // A tile's rows lie `side` rounded up to 12 more than a multiple of 32 words
 // apart: rows of the brush up to radius 6 then start in different banks.
 constexpr uint32_t kTilePitchMost = 204u;
@@ -82,6 +85,9 @@ constexpr uint32_t kTileBrushLanes = 8u;  // lanes that take one brush
 constexpr uint32_t kTileBrushes = 32u / kTileBrushLanes; // brushes a warp takes at a time
 constexpr uint32_t kTileMostPoints = 14u; // brush points per lane: up to radius 6
 constexpr uint32_t kTileMostRadius = 6u;
+// least starts' area, brushes of 4 and more, and lifetime: see erosion_tile_pays
+constexpr double kTileLeastArea = 1024.0 * 1024.0;
+constexpr uint32_t kTileLeastSteps = 30u;
 constexpr uint32_t kTileMostTiles = 48u * 1024u; // tile_scatter keeps a word of each in shared memory
 constexpr uint32_t kBinThreads = 256u;
 constexpr uint32_t kScanThreads = 1024u;
@@ -89,7 +95,8 @@ constexpr uint32_t kFinishThreads = 128u;
 // Few: what is left is few, or droplets that pile up in one place and would race there.
 constexpr uint32_t kFinishBlocks = 16u;
 constexpr int32_t kCellLimit = 1 << 29;
-constexpr int32_t kMoveUnits = 1 << 20;
+constexpr int32_t kMoveUnits = 1 << 21;
+static_assert(kCellLimit - 1 + int64_t { tile_threads(0u) } * kMoveUnits <= INT32_MAX, "a cell's sum leaves 32 bits");
 constexpr float kMoveLimit = static_cast<float>(kMoveUnits);
 // adding 1.5 * 2^23 leaves a float's nearest integer in its low bits (|x| < 2^22)
 constexpr float kMagic = 12582912.0f;
@@ -135,7 +142,7 @@ struct TileArgs {
 	uint32_t T, pitch;
 	uint32_t groups; // the starts of a job come in this many groups, one a phase
 	RainParams p;    // what all jobs have alike (all but BrushRadius, minWaterVolume and MaxSteps)
-	int32_t one1, minus1; // 1 and -1, unknown to the compiler: see pipe_add
+	int32_t minus1; // -1, unknown to the compiler: see pipe_add
 	TileStat* stat;
 	TileControl* ctl;
 	uint32_t* count[2]; // droplets per tile for an even / odd phase
@@ -157,13 +164,13 @@ __device__ __forceinline__ const TileJob& geom_of(const TileArgs& A, const uint3
 }
 
 // k of the unit 2^-k, or false where the tiles do not take the job: odd values, or a largest
-// height of more than 64 times the mean one (the unit is then 2^-25 of that or coarser)
+// height of more than 8 times the mean one (whose spacing as a float the unit then exceeds)
 __device__ __forceinline__ bool unit_of(const TileStat& s, const uint64_t cells, int& k) {
 	const float peak = __uint_as_float(s.peak);
-	if (s.odd || !(peak >= 1e-30f && peak <= 1e30f) || !(s.sum * 64.0 >= static_cast<double>(peak) * cells)) {
+	if (s.odd || !(peak >= 1e-30f && peak <= 1e30f) || !(s.sum * 8.0 >= static_cast<double>(peak) * cells)) {
 		return false;
 	}
-	k = 25 - ilogbf(peak);
+	k = 26 - ilogbf(peak);
 	return true;
 }
 __device__ __forceinline__ float power2(const int k) {
@@ -1008,15 +1015,13 @@ int tile_smem_attributes() {
 } // namespace
 
 // A tile for every SM out of the starts' areas (the droplets spread a little
-// past them), but no smaller than kTileLeast: a droplet moves a pixel a step,
-// so in small tiles it leaves after a few steps, takes many phases and strays
-// from the index order.  Measured, ms and RMS against the FP64 serial result:
-// a 3x3 x 512^2 chunk in tiles of 40, 48, 56, 64 3.26 / 3.61 / 3.95 / 4.49 and
-// 0.0012 / 0.0010 / 0.0009 / 0.0009; a 1024^2 field (brush 5, 64 steps) in tiles
-// of 56, 64, 72, 80, 96 4.53 / 4.53 / 4.63 / 4.40 / 5.07 and 0.0022 / 0.0021 /
-// 0.0019 / 0.0017 / 0.0016 (the reference GPU build 0.0010, its spread 0.0010);
-// sixteen 3x3 x 512^2 chunks in tiles of 80, 104, 128, 160, 200 19.6 / 18.7 /
-// 19.6 / 17.9 / 23.2 ms.
+// past them), but no smaller than kTileLeast: a droplet moves a pixel a step, so
+// in small tiles it leaves after a few steps and takes many phases, while later
+// droplets overtake it.  Measured, ms and RMS against the FP64 serial result, in
+// groups of 0.05 per pixel: a 1024^2 field (brush 5, 64 steps) in tiles of 80, 100,
+// 128, 160 5.70 / 5.53 / 7.16 / 9.33 and 0.00145 / 0.00131 / 0.00124 / 0.00121
+// (erosion.cu 9.00, 0.00123); a 2048^2 field in tiles of 100, 128, 160, 200 13.0 /
+// 12.9 / 13.1 / 14.4 and 0.00136 / 0.00128 / 0.00125 / 0.00123 (34.9, 0.00119).
 uint32_t erosion_tile_side(const ErosionJob* jobs, const uint32_t njobs) {
 	double area = 0.0, tiles = 0.0;
 	for (uint32_t j = 0u; j < njobs; j++) {
@@ -1043,20 +1048,36 @@ uint32_t erosion_tile_side(const ErosionJob* jobs, const uint32_t njobs) {
 	return tiles <= kTileMostTiles ? T : 0u;
 }
 
-// Brush points the droplets could erode in all.  From 10^9 on the tiles are the
-// better by far: erosion.cu against the tiles at 3x3 chunks, 1 droplet per
-// pixel, brush 5 and 60 steps 2.99 / 2.22 ms at 512^2 (1.1e9 points), 9.90 /
-// 4.04 at 1024^2 (4.3e9); 1500^2 field, brush 3, 40 steps 4.29 / 2.47 (1.35e9).
-// Below, the gain shrinks (384^2 1.97 / 1.90 at 0.6e9, 256^2 at 2.2 droplets per
-// pixel 2.21 / 3.40: few tiles hold starts) while small tiles follow the serial
-// order less closely (RMS against the FP64 serial result of 384^2 at 2 droplets
-// per pixel 0.0010 against 0.0005), so those calls keep to erosion.cu.
+namespace {
+
+// Whether a map's width keeps erosion.cu from taking brush rows as 16-byte blocks.
+bool no_rows(const ErosionJob* jobs, const uint32_t njobs) {
+	return std::any_of(jobs, jobs + njobs, [](const ErosionJob& j) { return (j.pitch & 3u) != 0u; });
+}
+
+} // namespace
+
+// Where the tiles are the better way and follow the serial order as closely.
+// A phase lasts as long as a tile's droplets take for their steps, however few
+// tiles hold any, so the tiles want wide starts' areas, and more so the fewer points
+// a brush has.  erosion.cu against the tiles, ms (3x3 chunks, 1 droplet per
+// pixel, 40 steps): 768^2 brush 5 3.78 / 4.52, 1024^2 brush 3 3.51 / 3.97, brush 4 4.76 /
+// 4.16, brush 5 6.13 / 4.70; fields at 0.95: 1448^2 brush 2 6.96 / 3.97, brush 3 6.28
+// / 4.30, 2048^2 brush 5 21.1 / 10.7.  Short lifetimes gain less, the launches'
+// share being larger (1024^2 brush 4 20 steps 2.39 / 2.45, 3000^2 brush 3 20 steps 4.08 / 4.22).
+// Without erosion.cu's rows (no_rows) the tiles gain more: 1025^2 brush 3 7.69 / 4.91; brushes of
+// 2 have no rows anyway.  Below 10^9 brush points either takes under 3 ms.
 bool erosion_tile_pays(const ErosionJob* jobs, const uint32_t njobs) {
-	double points = 0.0;
+	double points = 0.0, area = 0.0;
+	uint32_t radius = kTileMostRadius, steps = 0u;
 	for (uint32_t j = 0u; j < njobs; j++) {
 		points += static_cast<double>(jobs[j].count) * jobs[j].p.MaxSteps * jobs[j].brush_size;
+		area += jobs[j].start_area;
+		radius = std::min(radius, jobs[j].p.BrushRadius);
+		steps = std::max(steps, jobs[j].p.MaxSteps);
 	}
-	return points >= 1e9;
+	const bool wide_brush = radius >= (no_rows(jobs, njobs) ? 3u : 4u);
+	return points >= 1e9 && steps >= kTileLeastSteps && area >= (wide_brush ? kTileLeastArea : 2.0 * kTileLeastArea);
 }
 
 namespace {
@@ -1075,11 +1096,19 @@ TilePlan tile_plan(const ErosionJob* jobs, const uint32_t njobs, const uint32_t 
 		area += jobs[j].start_area;
 	}
 	TilePlan p;
-	// groups of at most 0.4 droplets per pixel, 0.25 where small tiles send droplets through many
-	// phases (production chunk, tiles of 40: RMS against the FP64 serial result 0.0022 in 7 groups
-	// and 0.0019 in 10, 3.65 and 3.72 ms; the reference GPU build 0.0013 with a spread of 0.0011)
-	const double per_group = T < 64u ? 0.25 : 0.4;
-	p.groups = static_cast<uint32_t>(std::min(16.0, std::max(4.0, std::ceil(droplets / area / per_group))));
+	// A droplet is under way for a few phases, and what then starts beside it is what departs from the
+	// serial order: groups of 0.05 droplets per pixel, of fewer the larger the map, where the kernels of
+	// erosion.cu hold fewer per pixel under way, too.  Measured, ms and RMS against the FP64 serial result,
+	// in groups of 0.2, 0.1, 0.05, 0.025, 0.0125 per pixel: a 4096^2 field (brush 5, 64 steps) 35.0 / 36.7 /
+	// 39.6 / 45.7 / 52.1 and 0.00142 / 0.00130 / 0.00125 / 0.00124 / 0.00123 (erosion.cu 136.6, 0.00120).
+	// Past 64 groups the launches cost more than the order gains: sixteen 3x3 x 512^2 chunks in 64 and 92
+	// groups 27.5 and 32.0 ms, 0.00043 either way (erosion.cu 59.5, 0.00042).
+	// Where erosion.cu goes without rows it is slower and follows the serial order more closely, and so do
+	// groups of half as many: a 1201^2 field (brush 4, 30 steps) in groups of 0.043, 0.025, 0.0125
+	// 3.45 / 4.16 / 7.50 and 0.00115 / 0.00112 / 0.00108 (erosion.cu 10.4, 0.00106).
+	const double wide = no_rows(jobs, njobs) ? 0.5 : 1.0;
+	const double per_group = wide * std::clamp(0.05 * 1024.0 / std::sqrt(area), 0.0125, 0.05);
+	p.groups = static_cast<uint32_t>(std::min(64.0 / wide, std::max(4.0, std::ceil(droplets / area / per_group))));
 	// a droplet that walks straight on crosses steps / T tiles; one that meanders comes back
 	p.phases = p.groups + 3u + (5u * steps + T - 1u) / T;
 	return p;
@@ -1125,7 +1154,6 @@ int erosion_tile_launch(const ErosionJob* host_jobs, const ErosionJob* jobs, con
 	A.T = T;
 	A.pitch = (T + 19u) / 32u * 32u + 12u;
 	A.p = host_jobs[0].p;
-	A.one1 = 1;
 	A.minus1 = -1;
 	A.groups = groups;
 	A.stat = reinterpret_cast<TileStat*>(ws + L.stat);
