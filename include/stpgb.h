@@ -214,7 +214,9 @@ STPGB_API int stpgb_nn_unmerge_host(const void* merged, uint32_t element_size, c
 
 /* Workspace bytes stpgb_shf_filter needs for a chunk of `nn`, `radius`, and
  * at most `max_items` distinct sample values in any filter window
- * (0 = the library maximum, 256). */
+ * (0 = the library maximum, 256).  A workspace begins at a multiple of 4 bytes;
+ * the few-values kernels and the row bands need a multiple of 8, and from
+ * another one every chunk takes the general slides. */
 STPGB_API int stpgb_shf_workspace_size(const stpgb_nn_info* nn, uint32_t radius,
 	uint32_t max_items, size_t* bytes);
 

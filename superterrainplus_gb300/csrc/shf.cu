@@ -827,6 +827,9 @@ int stpgb_shf_filter(const uint16_t* samplemap, const stpgb_nn_info* nn, uint32_
 		set_error("stpgb_shf_filter: workspace smaller than stpgb_shf_workspace_size");
 		return STPGB_ECAPACITY;
 	}
+	if ((reinterpret_cast<uintptr_t>(workspace) & 3u) != 0u) {
+		return inval("stpgb_shf_filter: workspace not aligned to 4 bytes");
+	}
 	const cudaStream_t s = as_stream(stream);
 	unsigned char* ws = static_cast<unsigned char*>(workspace);
 	ShfJob job;

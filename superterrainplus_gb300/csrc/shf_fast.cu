@@ -75,13 +75,13 @@ __device__ __forceinline__ bool list_tiles(const ShfJob& J, const uint32_t tr0, 
 	const uint32_t across = tc1 - tc0, tiles = (tr1 - tr0) * across, TC = tile_cols(J);
 	uint32_t last = kNoValue;
 	for (uint32_t i = t; i < tiles; i += n) {
-		const uint4* const slot = reinterpret_cast<const uint4*>(tile_slot(J, (tr0 + i / across) * TC + tc0 + i % across));
-		const uint4 a = slot[0], b = slot[1], c = slot[2];
-		const uint32_t held = a.x;
+		const uint2* const slot = reinterpret_cast<const uint2*>(tile_slot(J, (tr0 + i / across) * TC + tc0 + i % across));
+		const uint2 a = slot[1], b = slot[2], c = slot[3], d = slot[4];
+		const uint32_t held = slot[0].x;
 		if (held > most) {
 			return false;
 		}
-		const uint32_t words[kShfWideItems / 2u] = { a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y };
+		const uint32_t words[kShfWideItems / 2u] = { a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y };
 #pragma unroll
 		for (uint32_t k = 0u; k < kShfWideItems; k++) {
 			const uint32_t v = (words[k / 2u] >> (16u * (k & 1u))) & 0xFFFFu;

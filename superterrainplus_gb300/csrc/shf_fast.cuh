@@ -57,9 +57,11 @@ __device__ __forceinline__ uint64_t vn_bytes(const ShfJob& J) {
 __device__ __forceinline__ uint64_t tiles_bytes(const ShfJob& J) {
 	return 4ull * kSlotWords * tile_rows(J) * tile_cols(J);
 }
-// the others go the general slides without a palette
+// The others go the general slides without a palette: those read their workspace by words of four
+// bytes, these kernels by words of eight, and a caller's workspace may begin at any word.
 __device__ __forceinline__ bool has_palette(const ShfJob& J) {
-	return J.r <= kFastMaxRadius && tiles_bytes(J) <= vbuf_bytes(J) + vn_bytes(J);
+	return J.r <= kFastMaxRadius && (reinterpret_cast<uintptr_t>(J.vbuf) & 7u) == 0u
+		&& tiles_bytes(J) <= vbuf_bytes(J) + vn_bytes(J);
 }
 
 // A job's panels: panel p covers the columns [p * step, p * step + cols) of the
