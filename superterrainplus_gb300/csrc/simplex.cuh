@@ -20,13 +20,13 @@ __device__ __forceinline__ int floori(const float x) {
 
 // A corner's share from its weight before the power, half less its squared
 // distance, and the dot product of its gradient and offset.  Outside its reach
-// the weight is 0 and so is the product: no branch, which the lanes of a warp
-// would take differently.  The roundings are spelled out, here and in the
+// the share is 0, by a choice and not a branch, which the lanes of a warp would
+// take differently, nor by a weight of 0: a sample so far out that its offsets
+// or their product overflow has a share of 0 as well.  The roundings are spelled out, here and in the
 // weights and dot products, so that no change of the code around moves a height.
-__device__ __forceinline__ float corner(float w, const float dot) {
-	w = fmaxf(w, 0.0f);
-	w = __fmul_rn(w, w);
-	return __fmul_rn(__fmul_rn(w, w), dot);
+__device__ __forceinline__ float corner(const float w, const float dot) {
+	const float w2 = __fmul_rn(w, w);
+	return w <= 0.0f ? 0.0f : __fmul_rn(__fmul_rn(w2, w2), dot);
 }
 
 // Heights and splatmaps round the squared offset of the middle corner
