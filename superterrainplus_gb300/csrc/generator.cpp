@@ -17,6 +17,7 @@
 #include "shf.cuh"
 
 #include <algorithm>
+#include <functional>
 #include <memory>
 #include <mutex>
 #include <vector>
@@ -169,7 +170,9 @@ stpgb_nn_info make_nn(const uint32_t map[2], const uint32_t nn[2]) {
 // (STPNearestNeighbourTextureBuffer.cpp:94-111, chunk i at local
 // coordinate (i % nx, i / nx), STPChunk.cpp:71-73): of the merged map, the
 // columns [x0, x1) and rows [y0, y1).  One kernel where the GPU reads host
-// memory itself, else a 2D copy per chunk.
+// memory itself, else a 2D copy per chunk, and so where an array stands for two
+// places on the way out: the copies go one after the other, the kernel's blocks
+// in no order.
 template<typename T>
 int move_chunks(T* merged, T* const* chunks, const stpgb_nn_info& nn, const bool in, const uint32_t x0, const uint32_t y0,
 	const uint32_t x1, const uint32_t y1, cudaStream_t s) {
@@ -192,8 +195,13 @@ int move_chunks(T* merged, T* const* chunks, const stpgb_nn_info& nn, const bool
 		const uint32_t hp = static_cast<uint32_t>(row), dp = static_cast<uint32_t>(total_row);
 		rects.push_back(in ? HostRect { host, device, hp, dp, bytes, by - ay } : HostRect { device, host, dp, hp, bytes, by - ay });
 	}
+	std::vector<const T*> places(chunks, chunks + count);
+	std::sort(places.begin(), places.end(), std::less<const T*> {});
+	const bool apart = in || std::adjacent_find(places.begin(), places.end(), [&](const T* a, const T* b) {
+		return reinterpret_cast<uintptr_t>(b) - reinterpret_cast<uintptr_t>(a) < row * H;
+	}) == places.end();
 	const bool even = std::all_of(chunks, chunks + count, [](const T* p) { return (reinterpret_cast<uintptr_t>(p) & 1u) == 0u; });
-	if (row * H <= 0x7FFFFFFFull && total_row <= 0xFFFFFFFFull && even && host_memory_direct()) {
+	if (row * H <= 0x7FFFFFFFull && total_row <= 0xFFFFFFFFull && even && apart && host_memory_direct()) {
 		return copy_host_rects(rects.data(), static_cast<uint32_t>(rects.size()), s);
 	}
 	for (const HostRect& r : rects) {
