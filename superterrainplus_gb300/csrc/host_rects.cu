@@ -50,9 +50,11 @@ __global__ void __launch_bounds__(kRectThreads) rects_kernel(const RectList L) {
 } // namespace
 
 bool host_memory_direct() {
+	// through the host's page tables: a GPU that takes faults on such memory instead would move the
+	// caller's arrays to itself and back with every call
 	int dev = 0, yes = 0;
 	if (cudaGetDevice(&dev) != cudaSuccess
-		|| cudaDeviceGetAttribute(&yes, cudaDevAttrPageableMemoryAccess, dev) != cudaSuccess) {
+		|| cudaDeviceGetAttribute(&yes, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev) != cudaSuccess) {
 		cudaGetLastError();
 		return false;
 	}

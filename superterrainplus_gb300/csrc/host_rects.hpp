@@ -15,7 +15,7 @@ struct HostRect {
 	uint32_t src_pitch, dst_pitch, width, rows;
 };
 
-// Whether the current device reads and writes pageable host memory itself.
+// Whether the current device reads and writes pageable host memory itself, where it lies.
 bool host_memory_direct();
 // Enqueues the copies; host arrays must stay until the stream is waited for.
 int copy_host_rects(const HostRect* rects, uint32_t count, cudaStream_t stream);
