@@ -516,9 +516,7 @@ struct stpgb_batch {
 			}
 			const int erc = erosion_launch(nullptr, e, 1u, e.count, e.brush_size, s, G.lanes, false, G.dpg, G.rows,
 				erosion_rows_wide(G.min_radius), erosion_rows_atomic(G.min_radius, G.lanes), 1u, taken);
-			if (tiles) {
-				STPGB_CUDA_TRY(cudaFreeAsync(tiles, s));
-			}
+			STPGB_TRY(erosion_tile_release(tiles, s));
 			STPGB_TRY(erc);
 			const FormatJob& f = fmt_h[n];
 			STPGB_TRY(format_launch(f.in, f.in_pitch, f.out, f.out_pitch, f.W, f.H, s));

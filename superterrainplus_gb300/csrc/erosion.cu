@@ -1688,9 +1688,7 @@ int stpgb_hydraulic_erosion_ex(float* heightmap, const stpgb_nn_info* nn, const 
 	const int rc = erosion_launch(nullptr, job, 1u, count, brush_size, s, lanes, exact, dpg, rows,
 		erosion_rows_wide(setting->ErosionBrushRadius),
 		erosion_rows_atomic(setting->ErosionBrushRadius, lanes), 1u, gate);
-	if (tiles) {
-		STPGB_CUDA_TRY(cudaFreeAsync(tiles, s));
-	}
+	STPGB_TRY(erosion_tile_release(tiles, s));
 	return rc;
 }
 

@@ -166,10 +166,11 @@ int erosion_tile_launch(const ErosionJob* host_jobs, const ErosionJob* device_jo
 // kernels of such a launch
 uint32_t erosion_tile_kernels(const ErosionJob* jobs, uint32_t njobs, uint32_t side);
 // The same for one job with a workspace of the library's own, returned in `workspace` for the
-// caller to free on `stream` (cudaFreeAsync); null, and nothing launched, where the tiles do not
-// pay (unless `force`) or do not take the job, the stream is being captured or the workspace
-// cannot be had.
+// caller to give back on `stream` (erosion_tile_release); null, and nothing launched, where the
+// tiles do not pay (unless `force`) or do not take the job, the stream is being captured or the
+// workspace cannot be had.
 int erosion_tile_call(const ErosionJob& job, bool force, void** workspace, const uint32_t** taken, cudaStream_t stream);
+int erosion_tile_release(void* workspace, cudaStream_t stream);
 
 int format_launch(const float* in, uint64_t in_pitch, uint16_t* out, uint64_t out_pitch, uint32_t W, uint32_t H,
 	cudaStream_t stream);

@@ -1241,6 +1241,22 @@ constexpr int kPoolDevices = 64;
 std::mutex g_pool_mutex;
 cudaMemPool_t g_pool[kPoolDevices] = {};
 
+// Allocations are refused, and end the capture, while this thread or another captures a stream,
+// unless the thread says that it knows what it does: here they are on a stream that is not captured.
+class CaptureElsewhere {
+	cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+
+public:
+	CaptureElsewhere() {
+		cudaThreadExchangeStreamCaptureMode(&mode);
+	}
+	~CaptureElsewhere() {
+		cudaThreadExchangeStreamCaptureMode(&mode);
+	}
+	CaptureElsewhere(const CaptureElsewhere&) = delete;
+	CaptureElsewhere& operator=(const CaptureElsewhere&) = delete;
+};
+
 cudaMemPool_t tile_pool() {
 	int dev = 0;
 	if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kPoolDevices) {
@@ -1281,6 +1297,7 @@ int erosion_tile_call(const ErosionJob& job, const bool force, void** workspace,
 		cudaGetLastError();
 		return STPGB_OK;
 	}
+	const CaptureElsewhere guard;
 	const cudaMemPool_t pool = tile_pool();
 	void* ws = nullptr;
 	if (!pool || cudaMallocFromPoolAsync(&ws, erosion_tile_bytes(&job, 1u, T), pool, stream) != cudaSuccess) {
@@ -1293,6 +1310,14 @@ int erosion_tile_call(const ErosionJob& job, const bool force, void** workspace,
 		return rc;
 	}
 	*workspace = ws;
+	return STPGB_OK;
+}
+
+int erosion_tile_release(void* workspace, cudaStream_t stream) {
+	if (workspace) {
+		const CaptureElsewhere guard;
+		STPGB_CUDA_TRY(cudaFreeAsync(workspace, stream));
+	}
 	return STPGB_OK;
 }
 
