@@ -98,6 +98,8 @@ constexpr int32_t kCellLimit = 1 << 29;
 constexpr int32_t kMoveUnits = 1 << 21;
 static_assert(kCellLimit - 1 + int64_t { tile_threads(0u) } * kMoveUnits <= INT32_MAX, "a cell's sum leaves 32 bits");
 constexpr float kMoveLimit = static_cast<float>(kMoveUnits);
+// what others may put on a corner beside a droplet, in multiples of what it puts there itself
+constexpr int32_t kMostPuts = 3;
 // adding 1.5 * 2^23 leaves a float's nearest integer in its low bits (|x| < 2^22)
 constexpr float kMagic = 12582912.0f;
 constexpr int32_t kMagicBits = 0x4B400000;
@@ -696,11 +698,13 @@ __global__ void __launch_bounds__(tile_threads(Points), 1) tile_erode(const Tile
 							  s11 = atomicAdd(cells + at + pitch + 1, d11) - q11;
 				int32_t put = (d00 + d10) + (d01 + d11);
 				// What others have put on a corner since it was read is not put on it again, as a later
-				// droplet of the serial order would find it there: droplets that meet in a hollow, in
-				// lockstep in one warp even, would otherwise all fill it in full and raise a mound.
+				// droplet of the serial order would find it there, past kMostPuts times the droplet's own:
+				// droplets that meet in a hollow, in lockstep in one warp even, would otherwise all fill it in
+				// full and raise a mound.  (From the first on, what droplets put while others pass is taken
+				// back too: RMS of a 1024^2 field 0.00125, this way 0.00123, erosion.cu's 0.00122.)
 				if (max(max(s00, s10), max(s01, s11)) > 0) {
-					const int32_t e00 = min(max(s00, 0), d00), e10 = min(max(s10, 0), d10),
-								  e01 = min(max(s01, 0), d01), e11 = min(max(s11, 0), d11);
+					const int32_t e00 = min(max(s00 - kMostPuts * d00, 0), d00), e10 = min(max(s10 - kMostPuts * d10, 0), d10),
+								  e01 = min(max(s01 - kMostPuts * d01, 0), d01), e11 = min(max(s11 - kMostPuts * d11, 0), d11);
 					atomicAdd(cells + at, -e00);
 					atomicAdd(cells + at + 1, -e10);
 					atomicAdd(cells + at + pitch, -e01);
@@ -1101,14 +1105,14 @@ TilePlan tile_plan(const ErosionJob* jobs, const uint32_t njobs, const uint32_t 
 	// erosion.cu hold fewer per pixel under way, too.  Measured, ms and RMS against the FP64 serial result,
 	// in groups of 0.2, 0.1, 0.05, 0.025, 0.0125 per pixel: a 4096^2 field (brush 5, 64 steps) 35.0 / 36.7 /
 	// 39.6 / 45.7 / 52.1 and 0.00142 / 0.00130 / 0.00125 / 0.00124 / 0.00123 (erosion.cu 136.6, 0.00120).
-	// Past 64 groups the launches cost more than the order gains: sixteen 3x3 x 512^2 chunks in 64 and 92
-	// groups 27.5 and 32.0 ms, 0.00043 either way (erosion.cu 59.5, 0.00042).
+	// Past 48 groups the launches cost more than the order gains: sixteen 3x3 x 512^2 chunks in 48, 64 and
+	// 92 groups 24, 27.5 and 32.0 ms, 0.00043 each way (erosion.cu 59.5, 0.00042).
 	// Where erosion.cu goes without rows it is slower and follows the serial order more closely, and so do
 	// groups of half as many: a 1201^2 field (brush 4, 30 steps) in groups of 0.043, 0.025, 0.0125
 	// 3.45 / 4.16 / 7.50 and 0.00115 / 0.00112 / 0.00108 (erosion.cu 10.4, 0.00106).
 	const double wide = no_rows(jobs, njobs) ? 0.5 : 1.0;
 	const double per_group = wide * std::clamp(0.05 * 1024.0 / std::sqrt(area), 0.0125, 0.05);
-	p.groups = static_cast<uint32_t>(std::min(64.0 / wide, std::max(4.0, std::ceil(droplets / area / per_group))));
+	p.groups = static_cast<uint32_t>(std::min(48.0 / wide, std::max(4.0, std::ceil(droplets / area / per_group))));
 	// a droplet that walks straight on crosses steps / T tiles; one that meanders comes back
 	p.phases = p.groups + 3u + (5u * steps + T - 1u) / T;
 	return p;
