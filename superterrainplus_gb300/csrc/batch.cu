@@ -737,12 +737,12 @@ int stpgb_batch_create(const stpgb_batch_request* requests, uint32_t count, cons
 		STPGB_TRY(upload(b->grp[g].jobs, b->grp[g].h));
 	}
 	STPGB_TRY(upload(b->fmt_jobs, b->fmt_h));
-	// the tiles' workspaces, where the tiles pay and the budget has room for them
+	// the tiles' workspaces, where the tiles may be the faster way and the budget has room for them
 	for (uint32_t g = 0u; g < b->ngroups; g++) {
 		ErosionGroup& G = b->grp[g];
 		const uint32_t njobs = static_cast<uint32_t>(G.h.size()), side = erosion_tile_side(G.h.data(), njobs);
 		const size_t bytes = side ? erosion_tile_bytes(G.h.data(), njobs, side) : 0u;
-		if (side == 0u || !erosion_tile_pays(G.h.data(), njobs) || (hbm_budget != 0u && b->bytes + bytes > hbm_budget)) {
+		if (side == 0u || !erosion_tile_many(G.h.data(), njobs) || (hbm_budget != 0u && b->bytes + bytes > hbm_budget)) {
 			continue;
 		}
 		if (cudaMalloc(&G.tile_ws, bytes) != cudaSuccess) {
@@ -752,7 +752,7 @@ int stpgb_batch_create(const stpgb_batch_request* requests, uint32_t count, cons
 		}
 		b->bytes += bytes;
 		G.tile = side;
-		G.tiled = true;
+		G.tiled = erosion_tile_pays(G.h.data(), njobs); // the tuner measures
 		STPGB_TRY(erosion_tile_prepare(G.h.data(), njobs, side, G.tile_ws));
 	}
 	if (b->ngroups > 1u) {

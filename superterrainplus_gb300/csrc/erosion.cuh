@@ -152,7 +152,9 @@ ErosionChoice erosion_choice(uint32_t radius, uint32_t brush_size, double densit
 // Droplets that take more steps than this stay with the kernels above: a phase
 // of the tiles may hold a droplet until it has taken all of them.
 constexpr uint32_t kTileMaxSteps = 1024u;
-// Whether the tiles are the faster way for these jobs.
+// Whether these jobs are many enough to choose between the tiles and the kernels above, and whether
+// the tiles are the faster way.
+bool erosion_tile_many(const ErosionJob* jobs, uint32_t njobs);
 bool erosion_tile_pays(const ErosionJob* jobs, uint32_t njobs);
 // The tile side for a launch over these jobs, 0 where the tiles do not take one of them.
 uint32_t erosion_tile_side(const ErosionJob* jobs, uint32_t njobs);

@@ -1061,6 +1061,15 @@ bool no_rows(const ErosionJob* jobs, const uint32_t njobs) {
 
 } // namespace
 
+// Brush points enough that either way's time is worth choosing; below, either takes under 3 ms.
+bool erosion_tile_many(const ErosionJob* jobs, const uint32_t njobs) {
+	double points = 0.0;
+	for (uint32_t j = 0u; j < njobs; j++) {
+		points += static_cast<double>(jobs[j].count) * jobs[j].p.MaxSteps * jobs[j].brush_size;
+	}
+	return points >= 1e9;
+}
+
 // Where the tiles are the better way and follow the serial order as closely.
 // A phase lasts as long as a tile's droplets take for their steps, however few
 // tiles hold any, so the tiles want wide starts' areas, and more so the fewer points
@@ -1070,18 +1079,17 @@ bool no_rows(const ErosionJob* jobs, const uint32_t njobs) {
 // / 4.30, 2048^2 brush 5 21.1 / 10.7.  Short lifetimes gain less, the launches'
 // share being larger (1024^2 brush 4 20 steps 2.39 / 2.45, 3000^2 brush 3 20 steps 4.08 / 4.22).
 // Without erosion.cu's rows (no_rows) the tiles gain more: 1025^2 brush 3 7.69 / 4.91; brushes of
-// 2 have no rows anyway.  Below 10^9 brush points either takes under 3 ms.
+// 2 have no rows anyway.
 bool erosion_tile_pays(const ErosionJob* jobs, const uint32_t njobs) {
-	double points = 0.0, area = 0.0;
+	double area = 0.0;
 	uint32_t radius = kTileMostRadius, steps = 0u;
 	for (uint32_t j = 0u; j < njobs; j++) {
-		points += static_cast<double>(jobs[j].count) * jobs[j].p.MaxSteps * jobs[j].brush_size;
 		area += jobs[j].start_area;
 		radius = std::min(radius, jobs[j].p.BrushRadius);
 		steps = std::max(steps, jobs[j].p.MaxSteps);
 	}
 	const bool wide_brush = radius >= (no_rows(jobs, njobs) ? 3u : 4u);
-	return points >= 1e9 && steps >= kTileLeastSteps && area >= (wide_brush ? kTileLeastArea : 2.0 * kTileLeastArea);
+	return erosion_tile_many(jobs, njobs) && steps >= kTileLeastSteps && area >= (wide_brush ? kTileLeastArea : 2.0 * kTileLeastArea);
 }
 
 namespace {
