@@ -84,10 +84,10 @@ def requests(batch, rank):
                  DropletCount=DROPLETS, BrushRadius=BRUSH, Lifetime=LIFETIME) for n in range(batch)]
 
 
-# DRAM bytes of the production batch's erosion in tiles (16 requests, all its launches) from an ncu
-# capture, and the SM cycles a brush point's returning shared-memory add takes where nothing else runs
+# DRAM bytes of the production batch's erosion in tiles (16 requests, 53 phases of what an ncu capture of
+# three of them gives), and the SM cycles a brush point's returning shared-memory add takes where nothing else runs
 # (9.2 cycles per radius-4 brush of 45 points, brushes at random places of a tile)
-EROSION_TILES_DRAM_BYTES_PER_REQUEST = (1.89e9 + 0.46e9) / 16
+EROSION_TILES_DRAM_BYTES_PER_REQUEST = (2.5e9 + 0.1e9) / 16
 TILE_POINT_CYCLES = 9.2 / 45
 # kernels a batch run launches at most with its erosion on the L2: nine of the filter, noise, four
 # variant groups, format

@@ -356,7 +356,8 @@ STPGB_API int stpgb_hydraulic_erosion(float* heightmap, const stpgb_nn_info* nn,
  * STPGB_EROSION_EXACT_CLAMP erodes each point by compare-and-swap instead, so
  * racing droplets never remove more than a cell holds (closer to the serial
  * algorithm, slower).  Large calls on wide start areas (10^9 brush points and
- * 2^20 pixels or more, brushes of 3 and less 2^21, of 30 steps or more) erode
+ * 2^20 pixels or more, with brushes of 2, and of 3 on maps whose width 4
+ * divides, 2^21 pixels, and of 30 steps or more) erode
  * by default (lanes_per_droplet = 0, one droplet per group, no flag) in tiles
  * of the map held in shared memory instead; any call does so with
  * STPGB_EROSION_TILES, which explicit lanes or droplets per group and the other
@@ -371,7 +372,8 @@ enum { STPGB_EROSION_EXACT_CLAMP = 1, STPGB_EROSION_POINTWISE = 2, STPGB_EROSION
 
 /* The kernel variant the default (lanes_per_droplet = 0) of
  * stpgb_hydraulic_erosion_ex takes for a brush of `brush_radius` and
- * `droplets` over `area` pixels (the chunk the starts cover).  Racing
+ * `droplets` over `area` pixels (the chunk the starts cover), on calls that
+ * the tiles do not erode.  Racing
  * droplets packed densely enough dig channels without bound, and the faster
  * a droplet's brush update completes, the lower that density: up to 3
  * droplets per pixel and 1.5 in flight at once brush rows are taken (the
@@ -759,7 +761,7 @@ STPGB_API int stpgb_batch_tune(stpgb_batch* batch);
  * index 18*rows + 3*log2(lanes) + {0, 1, 2} for 1, 2, 4 droplets per group
  * (0 = not tried).  A group that erodes in shared-memory tiles
  * (STPGB_EROSION_TILES), because they were faster or, without tuning, because
- * its droplets are many, reports the fastest of these variants beside, which
+ * a single call of its droplets would, reports the fastest of these variants beside, which
  * erodes the maps the tiles do not take.  Any output pointer may be NULL. */
 STPGB_API int stpgb_batch_tuning(const stpgb_batch* batch, uint32_t* lanes_per_droplet,
 	uint32_t* droplets_per_group, uint32_t* vector_rows, float* erosion_ms);

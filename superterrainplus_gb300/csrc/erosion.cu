@@ -102,9 +102,9 @@ constexpr uint32_t kCasRetries = 16u;
 // One-lane droplets: a warp waits for its slowest droplet at every step, so it
 // takes fewer than 32 while the launch has no more than this many warps per SM
 // (half of what is resident, so that all stay in flight): a 64^2 chunk of 9011
-// droplets, 4 per warp, brush 4 and 50 steps, 1.85 -> 1.41 ms; 100^2, 8 per warp, brush 6
-// 5.08 -> 4.88; 128^2, 16 per warp, brush 2 0.52 -> 0.48, brush 3 1.01 -> 1.01.  Beyond that the warps
-// wait for each other instead (128^2, 4 per warp, 1.05).
+// droplets, 4 per warp, brush 4 and 50 steps, 2.05 -> 1.35 ms, brush 3 and 30 steps 0.79 -> 0.56;
+// 128^2 of 37684, 16 per warp, 30 steps, brush 3 0.96 -> 0.93, brush 2 0.50 either way.  Beyond that
+// the warps wait for each other instead (128^2, 4 per warp, 1.05).
 constexpr uint32_t kOneLaneWarpsPerSM = 24u;
 
 // G lanes (1, 2, 4, 8, 16 or 32) carry one droplet.  Every lane of a group
